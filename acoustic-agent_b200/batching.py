@@ -243,14 +243,14 @@ class RIRRenderer:
             plan.echo_prev.copy_(plan.echo_store)
             runtime.synthesize_batch(synth, plan.synth_workspace, stream=side, phase="raw")
             raw_done.record(side)
+            # the recursion's few blocks start before the trace takes every SM; the trace's persistent blocks
+            # that find no room beside them start when they end and take the chunks that are left then
+            runtime.synthesize_batch(synth, plan.synth_workspace, stream=side, phase="filter")
         main.wait_event(raw_done)
         with torch.cuda.stream(main):
             runtime.trace_batch([(plan.scenes[j.scene_index], j.spec, b) for j, b in zip(plan.jobs, plan.buffers)],
                                 plan.workspace, block_size=self.block_size, grid_blocks=self.grid_blocks,
                                 chunk_rays=self.chunk_rays, stack_entries=self.stack_entries, stream=main)
-        with torch.cuda.stream(side):
-            # the recursion runs as one-warp blocks beside the persistent trace blocks
-            runtime.synthesize_batch(synth, plan.synth_workspace, stream=side, phase="filter")
         main.wait_stream(side)
 
     def launch_pipelined(self, plan: Plan) -> None:

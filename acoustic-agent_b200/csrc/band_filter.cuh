@@ -1,160 +1,268 @@
 // The crossover recursion of bandlimit_band_signals (acoustic_agent/steam_rt.py
-// :3070-3083, :4131-4212) as a systolic warp: lane (unit, chain, stage) runs one
-// biquad section of an eight-pole low-pass and passes its float32 output one
-// lane up; section s runs kSkew samples behind section s-1.  A "unit" is one
-// band of one signal: bands 1-4 need two chains (the low-pass at the upper and
-// lower crossover, subtracted), bands 0 and 5 one.  Four units per warp.
+// :3070-3083, :4131-4212).  A band signal passes one or two eight-pole
+// low-passes (bands 1-4: the one at the upper crossover less the one at the
+// lower; band 0 the upper alone; band 5 the signal less the lower), each four
+// biquad sections in a row that hand on float32-rounded signals:
+//
+//     y0 = b0*x0 + b1*x1 + b2*x2 - a1*y1 - a2*y2, evaluated left to right.
 //
 // Included by every translation unit that band-limits signals; each of them is
 // compiled with -fmad=false, so the float64 arithmetic rounds operation by
-// operation like the reference's.
+// operation like the reference's and the outputs are its bits.
+//
+// What bounds it: the order of the operations is fixed, so a section's state
+// costs three dependent float64 operations per sample, (v - a1*y1) - a2*y2, of
+// 8.3 cycles each (25 cycles), whatever else runs beside it.  Everything that
+// is not this chain is therefore taken off it: one block carries kSignals
+// signals through all sections, with a warp for each job, in steps of
+// kStep samples between block barriers:
+//
+//   recursion warp s (one per scheduler): section s of every chain, one chain
+//       per lane; per sample a load of the input part v, the two products, the
+//       two differences, the rounding and a store -- nothing is exchanged
+//       between lanes and nothing waits inside a step but the chain itself;
+//   input warp(s) s: the input part v = (b0*x0 + b1*x1) + b2*x2 of section s,
+//       which does not depend on y, for all samples of a step in parallel;
+//   loader warp: the next steps' signals, by cp.async;
+//   output warp: the bands from the last section's outputs, coalesced.
+//
+// Section s runs two steps behind section s - 1 (input part, recursion).  One
+// RIR of 96,000 samples (10 chains), or eight of them on eight SMs, takes 1.70 ms
+// (35 cycles per sample) against 7.3 ms (150 cycles) for one warp per four bands
+// with a lane per section and shuffles between the sections.  The recursion
+// warp alone, without the others on its scheduler, runs at 29 cycles.
 #pragma once
 
 #include <cuda_runtime.h>
 
+#include <cstdint>
+#include <type_traits>
+
+#include "common.h"
+
 namespace ac {
 namespace {
 
-// One section of an eight-pole low-pass (steam_rt.py:4131-4146):
-//     y0 = b0*x0 + b1*x1 + b2*x2 - a1*y1 - a2*y2, evaluated left to right.
-// The input part ((b0*x0 + b1*x1) + b2*x2) does not depend on y, so it is
-// computed one sample ahead (`feed`); the per-sample recursion (`step`) is then
-// only (S - a1*y1) - a2*y2.  Same operations in the same order as the reference.
-struct Section {
-    double b0, b1, b2, a1, a2, x1, x2, y1, y2;
+constexpr int kSections = 4;
+// Signals per SM up to which each gets a block of its own.  A wide block (30 chains in the recursion lanes) takes 59
+// cycles per sample whatever it carries, a block of one signal 36, or 45 with two of them on an SM, which share the
+// float64 and conversion pipes; a third would make it 66.
+constexpr int kFilterNarrowPerSm = 2;
+constexpr int kFilterLag = 2 * kSections;   // steps between the input part of section 0 and the outputs
 
-    __device__ __forceinline__ double feed(double in) {
-        const double v = b0 * in + b1 * x1 + b2 * x2;
-        x2 = x1;
-        x1 = in;
-        return v;
-    }
-
-    __device__ __forceinline__ float step(double v) {
-        const double y0 = v - a1 * y1 - a2 * y2;
-        y2 = y1;
-        y1 = y0;
-        return static_cast<float>(y0);
-    }
+// One signal of a block: its band rows, `band_stride` apart (0: all bands share one row), and its outputs [6, n_len].
+struct FilterSignal {
+    const double *x;
+    int64_t band_stride;
+    float *out;
+    const double *crossover;   // [5 cutoffs][4 sections][5 coefficients]
+    int n_len;                 // 0: no signal in this place (the pointers are then another's, and nothing is read)
 };
 
-#ifndef AC_SYNTH_PREFETCH
-#define AC_SYNTH_PREFETCH 16
-#endif
-#ifndef AC_SYNTH_SKEW
-#define AC_SYNTH_SKEW 4
-#endif
-constexpr int kPrefetch = AC_SYNTH_PREFETCH;
-constexpr int kSkew = AC_SYNTH_SKEW;  // iterations between consecutive sections
-constexpr int kLag = kSkew * 3;  // section 3 runs kLag samples behind section 0
-static_assert(kSkew >= 3 && kLag + 2 <= kPrefetch, "the prefetch window must hold the lagged input");
-static_assert(kPrefetch >= 2, "section 0 reads its input two samples ahead");
+// kShared: the six bands share one input row, so the low-pass at a crossover is one chain for the two bands it
+// separates (5 chains per signal instead of 10).
+template <int kSignals, bool kShared>
+struct FilterShape {
+    static constexpr int kChains = kShared ? 5 : 10;
+    static constexpr int kInputs = kShared ? 1 : 6;
+    static constexpr int kLanes = kSignals * kChains;            // chains of the block
+    static constexpr int kWidth = kSignals * kInputs;            // input rows of the block
+    static constexpr int kXPitch = kWidth | 1;                   // odd pitches: a column has no bank conflicts
+    static constexpr int kYPitch = kLanes | 1;
+    static constexpr int kRowsAtOnce = 32 / kLanes;              // lanes of an input warp that share a chain
+    static constexpr int kInputWarps = kLanes > 16 ? 2 : 1;      // per section
+    // samples between two block barriers: a barrier and the refill of the recursion after it cost about 200 cycles;
+    // 64 (36.0 cycles per sample, 39.5 with 32) where two blocks of one signal then still fit an SM's shared memory
+    static constexpr int kStep = kSignals == 1 ? 64 : 32;
+    static constexpr int kRows = 4 * kStep;   // ring rows: the step being written, the one read and its history
+    static constexpr int kThreads = 32 * (kSections * (1 + kInputWarps) + 2);
+    static_assert(kLanes <= 32, "one chain per lane");
+};
 
-// Lane (unit, chain, stage): section `stage` works on sample it - kSkew*stage.
-// The float32 output it produces at iteration it is shuffled one lane up at
-// iteration it + 1 and consumed there at it + kSkew - 1 (as the input part of
-// its step at it + kSkew); the outputs are formed two iterations late and
-// written once per chunk of kPrefetch iterations.  So no instruction waits on
-// a shuffle issued in its own iteration, no store or bounds test sits in the
-// per-sample loop, and only the section's own y dependency is carried from one
-// iteration to the next.
-//
-// The body is branch-free: before a section's first real sample its input is
-// +0.0, and a section whose inputs and state are all +0.0 produces exactly +0.0
-// and keeps its state at +0.0 (every product is +0.0 or -0.0 and the sums come
-// out +0.0), so the steps while the pipeline fills change nothing.
-// The per-lane recursion of one warp.  `x` / `out_row` / `n_len` belong to the
-// lane's unit (band of one RIR); `co` points at the lane's section
-// coefficients.  `iterations` (the longest unit of the warp + kLag + 2) is
-// warp-uniform: every lane runs every iteration, so the shuffles stay full-warp.
-__device__ __forceinline__ void filter_units(const double *x, float *out_row, int n_len, bool valid_unit, int band,
-                                             const double *co, int iterations) {
-    const unsigned full = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31;
-    const int stage = lane & 3;
-    const int chain = (lane >> 2) & 1;
-    int cutoff;
-    bool active;
-    if (band == 0) { cutoff = 0; active = chain == 0; }
-    else if (band == 5) { cutoff = 4; active = chain == 0; }
-    else { cutoff = chain == 0 ? band : band - 1; active = true; }
-    active = active && valid_unit;
-    co += cutoff * 20 + stage * 5;
-    Section sec{co[0], co[1], co[2], co[3], co[4], 0.0, 0.0, 0.0, 0.0};
-    const bool emits = stage == 3 && chain == 0 && active;
-    const bool is_first = stage == 0;
-    const int mode = band == 0 ? 0 : (band == 5 ? 2 : 1);
+template <int kSignals, bool kShared>
+struct FilterSmem {
+    using Shape = FilterShape<kSignals, kShared>;
+    double x[Shape::kRows][Shape::kXPitch];
+    double v[kSections][2][Shape::kStep][Shape::kLanes];
+    float y[kSections][Shape::kRows][Shape::kYPitch];
+};
 
-    double ahead[kPrefetch], prev[kPrefetch];
+__device__ __forceinline__ void cp_async8_zfill(double *dst, const double *src, bool valid) {
+    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+    const int bytes = valid ? 8 : 0;   // past the end of the signal: zeros, and nothing is read
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(s), "l"(src), "r"(bytes) : "memory");
+}
+
+// All warps of the block meet here once per step.
+template <int kThreads>
+__device__ __forceinline__ void filter_barrier() {
+    __syncwarp();
+    asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+}
+
+// The whole block filters `signals[0 .. kSignals)`, which lie in shared memory.
+template <int kSignals, bool kShared>
+__device__ __forceinline__ void filter_block(const FilterSignal *signals, FilterSmem<kSignals, kShared> &m) {
+    using Shape = FilterShape<kSignals, kShared>;
+    constexpr int kLanes = Shape::kLanes, kChains = Shape::kChains, kInputs = Shape::kInputs;
+    constexpr int kStep = Shape::kStep, kRows = Shape::kRows;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int longest = 0;
 #pragma unroll
-    for (int u = 0; u < kPrefetch; ++u) {
-        ahead[u] = (valid_unit && u < n_len) ? __ldg(x + u) : 0.0;
-        prev[u] = 0.0;
+    for (int j = 0; j < kSignals; ++j) longest = max(longest, signals[j].n_len);
+    const int blocks = (longest + kStep - 1) / kStep;
+    {   // the history before the first sample is +0.0
+        unsigned *words = reinterpret_cast<unsigned *>(&m);
+        for (int i = threadIdx.x; i < static_cast<int>(sizeof(m) / 4); i += Shape::kThreads) words[i] = 0u;
     }
-    // q[d]: the value the previous section produced at iteration it - 1 - d (received through the
-    // shuffle issued one iteration after it was produced, so no shuffle result is used in the
-    // iteration that receives it); q[kSkew - 3] is this section's input two iterations ahead.
-    float q[kSkew - 2];
+    __syncthreads();
+
+    const int input_first = kSections, loader = kSections * (1 + Shape::kInputWarps);
+    auto load = [&](int k) {   // loader warp: step k's samples, lane = sample
 #pragma unroll
-    for (int i = 0; i < kSkew - 2; ++i) q[i] = 0.0f;
-    float y1f = 0.0f, y2f = 0.0f;   // this lane's float outputs of iterations it - 1 and it - 2
-    float lower2 = 0.0f;            // the lower chain's output of iteration it - 2
-    // input parts of the first two samples (their inputs are ahead[0], ahead[1] for section 0 and +0.0 for the
-    // later sections); each iteration then forms the input part two samples ahead, so that its dependent
-    // chain (conversion, products, sums) has a whole iteration to complete before the recursion needs it
-    double v = sec.feed(is_first ? ahead[0] : 0.0);
-    double v_next = sec.feed(is_first ? ahead[1] : 0.0);
-    for (int base = 0; base < iterations; base += kPrefetch) {
-        double next[kPrefetch];
-        float emitted[kPrefetch];   // this chunk's outputs, written after the chunk (off the recursion's path)
+        for (int jh = 0; jh < kSignals * (kStep / 32); ++jh) {
+            const int j = jh / (kStep / 32), n = k * kStep + jh % (kStep / 32) * 32 + lane;
+            const FilterSignal sg = signals[j];
+            const bool valid = n < sg.n_len;
+            const double *p = sg.x + (valid ? n : 0);
 #pragma unroll
-        for (int u = 0; u < kPrefetch; ++u) {
-            const int m = base + kPrefetch + u;
-            next[u] = (valid_unit && m < n_len) ? __ldg(x + m) : 0.0;
+            for (int b = 0; b < kInputs; ++b)
+                cp_async8_zfill(&m.x[n & (kRows - 1)][j * kInputs + b], p + b * sg.band_stride, valid);
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (warp == loader) {
+        load(0);
+        load(1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");   // step 0's samples are there
+    }
+    filter_barrier<Shape::kThreads>();
+    const int steps = blocks + kFilterLag;
+    // chain of this lane: signal, cutoff and input row
+    const bool recursion = warp < kSections;
+    const int slot = recursion ? lane : lane % kLanes;
+    const bool has_chain = recursion ? lane < kLanes : lane < Shape::kRowsAtOnce * kLanes;
+    const int chain_signal = has_chain ? slot / kChains : 0, chain = has_chain ? slot % kChains : 0;
+    const int cutoff = chain < 5 ? chain : chain - 5;
+    const int input = kShared ? chain_signal : chain_signal * kInputs + (chain < 5 ? chain : chain - 4);
+
+    if (recursion) {
+        const int s = warp;
+        const double *co = signals[chain_signal].crossover + cutoff * 20 + s * 5;
+        const double a1 = co[3], a2 = co[4];
+        double y1 = 0.0, y2 = 0.0;
+        for (int i = 0; i < steps; ++i) {
+            const int k = i - 1 - 2 * s;
+            if (k >= 0 && k < blocks && has_chain) {
+                const double *vp = &m.v[s][k & 1][0][lane];
+                float *yp = &m.y[s][(k * kStep) & (kRows - 1)][lane];
+                double v[8], next[8];
 #pragma unroll
-        for (int u = 0; u < kPrefetch; ++u) {
-            const int it = base + u;
-            const float y = sec.step(v);   // the recursion: the only chain carried from one iteration to the next
-            // exchange the outputs of the previous iteration, already rounded to float32
-            const float sent = __shfl_up_sync(full, y1f, 1);
-            const float lower = __shfl_down_sync(full, y1f, 4);
+                for (int u = 0; u < 8; ++u) v[u] = vp[u * kLanes];
 #pragma unroll
-            for (int i = kSkew - 3; i > 0; --i) q[i] = q[i - 1];
-            q[0] = sent;
-            // input part of iteration it + 2: section 0 reads the prefetched signal, later sections the
-            // value their predecessor produced at it + 2 - kSkew, received at it - 1 (q[kSkew - 3])
-            const double in_2 = is_first ? (u + 2 < kPrefetch ? ahead[u + 2] : next[u + 2 - kPrefetch])
-                                         : static_cast<double>(q[kSkew - 3]);
-            v = v_next;
-            v_next = sec.feed(in_2);
-            // output of iteration it - 2; x[it - 2 - kLag] is still in registers from the prefetch
-            const int k = u - 2 - kLag;
-            const double x_n = k >= 0 ? ahead[k] : prev[k + kPrefetch];
-            const float band5 = static_cast<float>(x_n - static_cast<double>(y2f));
-            emitted[u] = mode == 0 ? y2f : (mode == 2 ? band5 : y2f - lower2);
-            lower2 = lower;
-            y2f = y1f;
-            y1f = y;
-        }
-        // iteration base + u produced output sample base + u - 2 - kLag
-        const int first = base - 2 - kLag;
-        if (emits) {
-            if (first >= 0 && first + kPrefetch <= n_len) {
+                for (int base = 0; base < kStep; base += 8) {
+                    if (base + 8 < kStep) {
 #pragma unroll
-                for (int u = 0; u < kPrefetch; ++u) out_row[first + u] = emitted[u];
-            } else {
+                        for (int u = 0; u < 8; ++u) next[u] = vp[(base + 8 + u) * kLanes];
+                    }
 #pragma unroll
-                for (int u = 0; u < kPrefetch; ++u)
-                    if (first + u >= 0 && first + u < n_len) out_row[first + u] = emitted[u];
+                    for (int u = 0; u < 8; ++u) {
+                        const double y0 = v[u] - a1 * y1 - a2 * y2;
+                        y2 = y1;
+                        y1 = y0;
+                        yp[(base + u) * Shape::kYPitch] = static_cast<float>(y0);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) v[u] = next[u];
+                }
             }
+            filter_barrier<Shape::kThreads>();
         }
+    } else if (warp < loader) {
+        const int s = (warp - input_first) / Shape::kInputWarps, part = (warp - input_first) % Shape::kInputWarps;
+        const double *co = signals[chain_signal].crossover + cutoff * 20 + s * 5;
+        const double b0 = co[0], b1 = co[1], b2 = co[2];
+        // a lane takes kRun samples in a row of its chain: each value is loaded and widened once, and all loads of a
+        // step are issued before the first of them is used (one after another, a step of them took as long as the
+        // recursion itself)
+        constexpr int kShare = kStep / Shape::kInputWarps;   // samples of this warp per step
+        constexpr int kRun = (kShare + Shape::kRowsAtOnce - 1) / Shape::kRowsAtOnce;
+        const int run = lane / kLanes * kRun, first = part * kShare + run;
+        for (int i = 0; i < steps; ++i) {
+            const int k = i - 2 * s;
+            if (k >= 0 && k < blocks && has_chain) {
+                const int n = k * kStep + first;
+                double *vp = &m.v[s][k & 1][first][slot];
+                double x[kRun + 2];   // x[u + 2]: sample n + u
+                if (s == 0) {
 #pragma unroll
-        for (int u = 0; u < kPrefetch; ++u) {
-            prev[u] = ahead[u];
-            ahead[u] = next[u];
+                    for (int u = 0; u < kRun + 2; ++u)
+                        x[u] = run + u - 2 < kShare ? m.x[(n + u - 2) & (kRows - 1)][input] : 0.0;
+                } else {
+                    float f[kRun + 2];
+#pragma unroll
+                    for (int u = 0; u < kRun + 2; ++u)
+                        f[u] = run + u - 2 < kShare ? m.y[s - 1][(n + u - 2) & (kRows - 1)][slot] : 0.0f;
+#pragma unroll
+                    for (int u = 0; u < kRun + 2; ++u) x[u] = static_cast<double>(f[u]);
+                }
+                double v[kRun];
+#pragma unroll
+                for (int u = 0; u < kRun; ++u) v[u] = b0 * x[u + 2] + b1 * x[u + 1] + b2 * x[u];
+#pragma unroll
+                for (int u = 0; u < kRun; ++u)
+                    if (run + u < kShare) vp[u * kLanes] = v[u];
+            }
+            filter_barrier<Shape::kThreads>();
+        }
+    } else if (warp == loader) {
+        for (int i = 0; i < steps; ++i) {
+            load(i + 2);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");   // step i + 1's samples are there
+            filter_barrier<Shape::kThreads>();
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    } else {
+        for (int i = 0; i < steps; ++i) {
+            const int k = i - kFilterLag;
+            if (k >= 0) {
+#pragma unroll
+                for (int jh = 0; jh < kSignals * (kStep / 32); ++jh) {
+                    const int j = jh / (kStep / 32), n = k * kStep + jh % (kStep / 32) * 32 + lane;
+                    const FilterSignal sg = signals[j];
+                    if (n < sg.n_len) {
+                        const double x5 = __ldg(sg.x + 5 * sg.band_stride + n);
+                        const float *y = &m.y[kSections - 1][n & (kRows - 1)][j * kChains];
+                        const float *lower = kShared ? y : y + 5;   // lower[b - 1]: band b's lower low-pass
+                        float *out = sg.out + n;
+                        const size_t row = static_cast<size_t>(sg.n_len);
+                        out[0] = y[0];
+#pragma unroll
+                        for (int b = 1; b < 5; ++b) out[b * row] = y[b] - lower[b - 1];
+                        out[5 * row] = static_cast<float>(x5 - static_cast<double>(lower[4]));
+                    }
+                }
+            }
+            filter_barrier<Shape::kThreads>();
         }
     }
+}
+
+// Opts a filter kernel into its dynamic shared memory on the current device.
+template <class Kernel>
+inline int filter_smem(Kernel kernel, size_t bytes) {
+    AC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+    return AC_OK;
+}
+
+// Calls launch(std::integral_constant<int, signals per block>, blocks) for a batch of `count` signals.
+template <int kWide, class Launch>
+inline int with_filter_signals(int count, Launch launch) {
+    int device = 0, sms = 0;
+    AC_CUDA_TRY(cudaGetDevice(&device));
+    AC_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    if (count <= kFilterNarrowPerSm * sms) return launch(std::integral_constant<int, 1>{}, count);
+    return launch(std::integral_constant<int, kWide>{}, (count + kWide - 1) / kWide);
 }
 
 }  // namespace

@@ -34,8 +34,8 @@
 // which is why the delays must be at least 128 samples (see check_fdn).
 //
 // ac_late_tail restates the rest of _render_parametric_fdn_late_reverb
-// (:2588-2640): bandlimit_band_signals of the impulse (the systolic crossover
-// filter of band_filter.cuh, bit-identical), then one block per (RIR, band)
+// (:2588-2640): bandlimit_band_signals of the impulse (the crossover filter
+// of band_filter.cuh, bit-identical), then one block per (RIR, band)
 // measures the traced power at the anchor (_late_tail_start_power,
 // :2473-2497), scales the FDN band to the target energy and writes the
 // equal-power crossfade.  Its sums run in a fixed order but not numpy's
@@ -348,19 +348,23 @@ struct LateJobDev {
     int32_t rate_index;
 };
 
-// bandlimit_band_signals(np.repeat(raw_fdn[None, :], 6, axis=0)): every band
-// filters the same impulse.  Unit = job * 6 + band, four per warp.
-__global__ void __launch_bounds__(32) late_band_kernel(const LateJobDev *jobs, int num_units, int longest,
-                                                       const __grid_constant__ ac_synth_batch_config cfg) {
-    const int lane = threadIdx.x & 31;
-    const int unit = blockIdx.x * 4 + (lane >> 3);
-    const bool valid_unit = unit < num_units;
-    const LateJobDev &job = jobs[valid_unit ? unit / 6 : 0];
-    const int band = valid_unit ? unit % 6 : 0;
-    const int n_len = valid_unit ? job.num_samples : 0;
-    filter_units(job.fdn, job.bands + static_cast<int64_t>(band) * job.num_samples, n_len, valid_unit, band,
-                 cfg.crossover[job.rate_index], longest + kLag + 2);
+// bandlimit_band_signals(np.repeat(raw_fdn[None, :], 6, axis=0)): every band filters the same impulse.
+template <int kSignals>
+__global__ void __launch_bounds__(FilterShape<kSignals, true>::kThreads)
+    late_band_kernel(const LateJobDev *jobs, int num_jobs, const __grid_constant__ ac_synth_batch_config cfg) {
+    extern __shared__ __align__(16) unsigned char filter_smem_raw[];
+    __shared__ FilterSignal signals[kSignals];
+    if (threadIdx.x < kSignals) {
+        const int first = static_cast<int>(blockIdx.x) * kSignals, j = first + threadIdx.x;
+        const LateJobDev &job = jobs[j < num_jobs ? j : first];
+        signals[threadIdx.x] = FilterSignal{job.fdn, 0, job.bands, cfg.crossover[job.rate_index],
+                                            j < num_jobs ? job.num_samples : 0};
+    }
+    __syncthreads();
+    filter_block<kSignals, true>(signals, *reinterpret_cast<FilterSmem<kSignals, true> *>(filter_smem_raw));
 }
+
+constexpr int kLateWide = 6;   // tails per filter block in a large batch: 30 chains, one per recursion lane
 
 constexpr int kMixThreads = 256;
 
@@ -584,7 +588,6 @@ int ensure_fdn_smem(int bytes) {
 struct LateLayout {
     size_t jobs, bands, total;
     int64_t band_floats;
-    int longest;
 };
 
 int check_late(const ac_late_tail_job *jobs, int32_t num_jobs, const ac_synth_batch_config *cfg, bool need_buffers,
@@ -613,7 +616,6 @@ int check_late(const ac_late_tail_job *jobs, int32_t num_jobs, const ac_synth_ba
         if (need_buffers && (!job.traced || !job.fdn || !job.out || !job.fdn_component || !job.stats))
             return fail(AC_ERR_INVALID, "late tail job %d: null buffer", j);
         l.band_floats += static_cast<int64_t>(align256(6 * static_cast<size_t>(N) * sizeof(float)) / sizeof(float));
-        l.longest = std::max(l.longest, N);
     }
     size_t off = 0;
     l.jobs = off;  off = align256(off + static_cast<size_t>(num_jobs) * sizeof(LateJobDev));
@@ -747,8 +749,17 @@ extern "C" int ac_late_tail(const ac_late_tail_job *jobs, int32_t num_jobs, cons
     if (!host_staging) AC_CUDA_TRY(cudaStreamSynchronize(stream));
     const ac::LateJobDev *d_jobs = reinterpret_cast<const ac::LateJobDev *>(ws + l.jobs);
     const int units = 6 * num_jobs;
-    ac::late_band_kernel<<<(units + 3) / 4, 32, 0, stream>>>(d_jobs, units, l.longest, *config);
-    AC_CUDA_TRY(cudaGetLastError());
+    const int frc = ac::with_filter_signals<ac::kLateWide>(num_jobs, [&](auto signals, int blocks) -> int {
+        constexpr int kSignals = decltype(signals)::value;
+        const size_t smem = sizeof(ac::FilterSmem<kSignals, true>);
+        const int rc2 = ac::filter_smem(ac::late_band_kernel<kSignals>, smem);
+        if (rc2 != AC_OK) return rc2;
+        ac::late_band_kernel<kSignals>
+            <<<blocks, ac::FilterShape<kSignals, true>::kThreads, smem, stream>>>(d_jobs, num_jobs, *config);
+        AC_CUDA_TRY(cudaGetLastError());
+        return AC_OK;
+    });
+    if (frc != AC_OK) return frc;
     ac::late_mix_kernel<<<units, ac::kMixThreads, 0, stream>>>(d_jobs, *config);
     AC_CUDA_TRY(cudaGetLastError());
     return AC_OK;

@@ -8,12 +8,8 @@
 // float64, and each biquad section hands its successor a float32-rounded signal.
 //
 // The raw band signals are materialised first by a fully parallel kernel.  The
-// recursion itself is sequential in time, so parallelism comes from elsewhere
-// (band_filter.cuh): one warp is a systolic array of 8 four-section low-pass chains.  Lane
-// (unit, chain, stage) runs one biquad section and passes its float32 output
-// one lane up; section s runs kSkew samples behind section s-1.  A "unit" is
-// one band of one RIR: bands 1-4 need two chains (the low-pass at the upper
-// and lower crossover, subtracted), bands 0 and 5 one.  Four units per warp.
+// recursion itself is sequential in time (band_filter.cuh): one block filters
+// one RIR, or kFilterWide of them in a large batch.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -31,6 +27,7 @@ namespace {
 
 constexpr int kSynthBands = 6;
 constexpr double kSynthPi = 3.141592653589793;
+constexpr int kFilterWide = 3;   // RIRs per filter block in a large batch: 30 chains, one per recursion lane
 
 struct SynthArgs {
     double crossover[100];
@@ -120,18 +117,20 @@ __global__ void synth_raw_kernel(const double *amps, const double *air, const do
     }
 }
 
-__global__ void __launch_bounds__(128) synth_filter_kernel(const double *raw, const __grid_constant__ SynthArgs a,
-                                                           float *out) {
-    const int lane = threadIdx.x & 31;
-    const int warp = static_cast<int>((blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5);
-    const int unit = warp * 4 + (lane >> 3);
-    const int units = a.num_rirs * kSynthBands;
-    const bool valid_unit = unit < units;
-    const int band = valid_unit ? unit % kSynthBands : 0;
-    const int N = a.num_bins * a.spb;
-    const double *x = raw + static_cast<size_t>(valid_unit ? unit : 0) * static_cast<size_t>(N);
-    float *out_row = out + static_cast<size_t>(valid_unit ? unit : 0) * static_cast<size_t>(N);
-    filter_units(x, out_row, N, valid_unit, band, a.crossover, N + kLag + 2);
+template <int kSignals>
+__global__ void __launch_bounds__(FilterShape<kSignals, false>::kThreads)
+    synth_filter_kernel(const double *raw, const __grid_constant__ SynthArgs a, float *out) {
+    extern __shared__ __align__(16) unsigned char filter_smem_raw[];
+    __shared__ FilterSignal signals[kSignals];
+    if (threadIdx.x < kSignals) {
+        const int j = static_cast<int>(blockIdx.x) * kSignals + threadIdx.x;
+        const bool real = j < a.num_rirs;
+        const int N = a.num_bins * a.spb;
+        const size_t row = static_cast<size_t>(real ? j : 0) * kSynthBands * static_cast<size_t>(N);
+        signals[threadIdx.x] = FilterSignal{raw + row, N, out + row, a.crossover, real ? N : 0};
+    }
+    __syncthreads();
+    filter_block<kSignals, false>(signals, *reinterpret_cast<FilterSmem<kSignals, false> *>(filter_smem_raw));
 }
 
 // ---- ragged batches (ac_synthesize_batch) ----------------------------------
@@ -227,26 +226,38 @@ __global__ void synth_batch_raw_kernel(const SynthJobDev *jobs, const int64_t *s
     }
 }
 
-// Warp w runs units[4w .. 4w+3] (job << 3 | band, or -1); units are ordered
-// longest job first, so the four units of a warp have similar lengths.
-__global__ void __launch_bounds__(32) synth_batch_filter_kernel(const SynthJobDev *jobs, const int32_t *units,
-                                                                int num_units,
-                                                                const __grid_constant__ ac_synth_batch_config cfg,
-                                                                const double *raw) {
-    const int lane = threadIdx.x & 31;
-    const int warp = static_cast<int>((blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5);
-    const int slot = warp * 4 + (lane >> 3);
-    const int code = slot < num_units ? __ldg(units + slot) : -1;
-    const bool valid_unit = code >= 0;
-    const int j = valid_unit ? code >> 3 : 0;
-    const int band = valid_unit ? code & 7 : 0;
-    const SynthJobDev &job = jobs[j];
-    const int n_len = valid_unit ? job.num_bins * job.spb : 0;
-    const int longest = __reduce_max_sync(0xFFFFFFFFu, static_cast<unsigned>(n_len));
-    const double *x = raw + 6 * job.samples + static_cast<int64_t>(band) * n_len;
-    float *out_row = job.band_irs + static_cast<int64_t>(band) * n_len;
-    filter_units(x, out_row, n_len, valid_unit, band, cfg.crossover[valid_unit ? job.rate_index : 0],
-                 longest + kLag + 2);
+// Block b filters the jobs order[kSignals * b ...] (-1: none); the order is longest job first, so the jobs of a block
+// have similar lengths.
+template <int kSignals>
+__global__ void __launch_bounds__(FilterShape<kSignals, false>::kThreads)
+    synth_batch_filter_kernel(const SynthJobDev *jobs, const int32_t *order,
+                              const __grid_constant__ ac_synth_batch_config cfg, const double *raw) {
+    extern __shared__ __align__(16) unsigned char filter_smem_raw[];
+    __shared__ FilterSignal signals[kSignals];
+    if (threadIdx.x < kSignals) {
+        const int first = order[static_cast<int>(blockIdx.x) * kSignals];
+        const int j = order[static_cast<int>(blockIdx.x) * kSignals + threadIdx.x];
+        const SynthJobDev &job = jobs[j >= 0 ? j : first];
+        const int N = job.num_bins * job.spb;
+        signals[threadIdx.x] = FilterSignal{raw + 6 * job.samples, N, job.band_irs, cfg.crossover[job.rate_index],
+                                            j >= 0 ? N : 0};
+    }
+    __syncthreads();
+    filter_block<kSignals, false>(signals, *reinterpret_cast<FilterSmem<kSignals, false> *>(filter_smem_raw));
+}
+
+int launch_batch_filter(const SynthJobDev *jobs, const int32_t *order, int num_jobs, const ac_synth_batch_config &cfg,
+                        const double *raw, cudaStream_t stream) {
+    return with_filter_signals<kFilterWide>(num_jobs, [&](auto signals, int blocks) -> int {
+        constexpr int kSignals = decltype(signals)::value;
+        const size_t smem = sizeof(FilterSmem<kSignals, false>);
+        const int rc = filter_smem(synth_batch_filter_kernel<kSignals>, smem);
+        if (rc != AC_OK) return rc;
+        synth_batch_filter_kernel<kSignals>
+            <<<blocks, FilterShape<kSignals, false>::kThreads, smem, stream>>>(jobs, order, cfg, raw);
+        AC_CUDA_TRY(cudaGetLastError());
+        return AC_OK;
+    });
 }
 
 }  // namespace
@@ -305,12 +316,15 @@ int enqueue_synthesis(const float *echograms, const ac_synth_params *p, float *b
     const int raw_grid = static_cast<int>(std::min<size_t>((samples + 255) / 256, 65536));
     synth_raw_kernel<<<raw_grid, 256, 0, stream>>>(amps, air_table, wtab, noise, stride, a, raw);
     AC_CUDA_TRY(cudaGetLastError());
-    const int units = p->num_rirs * 6;
-    const int warps = (units + 3) / 4;
-    const int threads = 32;  // one warp per block: spread the sequential chains over all SMs
-    synth_filter_kernel<<<warps, threads, 0, stream>>>(raw, a, band_irs);
-    AC_CUDA_TRY(cudaGetLastError());
-    return AC_OK;
+    return with_filter_signals<kFilterWide>(p->num_rirs, [&](auto signals, int blocks) -> int {
+        constexpr int kSignals = decltype(signals)::value;
+        const size_t smem = sizeof(FilterSmem<kSignals, false>);
+        const int rc = filter_smem(synth_filter_kernel<kSignals>, smem);
+        if (rc != AC_OK) return rc;
+        synth_filter_kernel<kSignals><<<blocks, FilterShape<kSignals, false>::kThreads, smem, stream>>>(raw, a, band_irs);
+        AC_CUDA_TRY(cudaGetLastError());
+        return AC_OK;
+    });
 }
 
 }  // namespace
@@ -336,9 +350,9 @@ namespace ac {
 namespace {
 
 struct SynthBatchLayout {
-    size_t jobs, cell_prefix, sample_prefix, units, table_end, amps, air, raw, total;
+    size_t jobs, cell_prefix, sample_prefix, order, table_end, amps, air, raw, total;
     int64_t cells, samples;
-    int32_t num_units;
+    int32_t num_slots;   // jobs rounded up to whole blocks of kFilterWide
 };
 
 int check_batch(const ac_synth_job *jobs, int32_t num_jobs, const ac_synth_batch_config *cfg, bool need_buffers,
@@ -371,12 +385,12 @@ int check_batch(const ac_synth_job *jobs, int32_t num_jobs, const ac_synth_batch
         l.cells += 6 * static_cast<int64_t>(job.num_bins);
         l.samples += N;
     }
-    l.num_units = static_cast<int32_t>((6 * static_cast<int64_t>(num_jobs) + 3) / 4 * 4);
+    l.num_slots = (num_jobs + kFilterWide - 1) / kFilterWide * kFilterWide;
     size_t off = 0;
     l.jobs = off;          off = align256(off + static_cast<size_t>(num_jobs) * sizeof(SynthJobDev));
     l.cell_prefix = off;   off = align256(off + (static_cast<size_t>(num_jobs) + 1) * sizeof(int64_t));
     l.sample_prefix = off; off = align256(off + (static_cast<size_t>(num_jobs) + 1) * sizeof(int64_t));
-    l.units = off;         off = align256(off + static_cast<size_t>(l.num_units) * sizeof(int32_t));
+    l.order = off;         off = align256(off + static_cast<size_t>(l.num_slots) * sizeof(int32_t));
     l.table_end = off;
     l.amps = off;          off = align256(off + static_cast<size_t>(l.cells) * sizeof(double));
     l.air = off;           off = align256(off + static_cast<size_t>(l.cells) * sizeof(double));
@@ -416,14 +430,10 @@ int synth_batch_phase(const ac_synth_job *jobs, int32_t num_jobs, const ac_synth
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
     unsigned char *ws = static_cast<unsigned char *>(workspace);
     const ac::SynthJobDev *d_jobs = reinterpret_cast<const ac::SynthJobDev *>(ws + l.jobs);
-    const int32_t *d_units = reinterpret_cast<const int32_t *>(ws + l.units);
+    const int32_t *d_order = reinterpret_cast<const int32_t *>(ws + l.order);
     double *raw = reinterpret_cast<double *>(ws + l.raw);
     if (!raw_phase) {
-        if (filter_phase) {
-            ac::synth_batch_filter_kernel<<<l.num_units / 4, 32, 0, stream>>>(d_jobs, d_units, l.num_units, *config, raw);
-            AC_CUDA_TRY(cudaGetLastError());
-        }
-        return AC_OK;
+        return filter_phase ? ac::launch_batch_filter(d_jobs, d_order, num_jobs, *config, raw, stream) : AC_OK;
     }
     std::vector<unsigned char> local;
     unsigned char *host = static_cast<unsigned char *>(host_staging);
@@ -434,7 +444,7 @@ int synth_batch_phase(const ac_synth_job *jobs, int32_t num_jobs, const ac_synth
     ac::SynthJobDev *dev_jobs = reinterpret_cast<ac::SynthJobDev *>(host + l.jobs);
     int64_t *cell_prefix = reinterpret_cast<int64_t *>(host + l.cell_prefix);
     int64_t *sample_prefix = reinterpret_cast<int64_t *>(host + l.sample_prefix);
-    int32_t *units = reinterpret_cast<int32_t *>(host + l.units);
+    int32_t *order = reinterpret_cast<int32_t *>(host + l.order);
     int64_t cells = 0, samples = 0;
     for (int32_t j = 0; j < num_jobs; ++j) {
         const ac_synth_job &in = jobs[j];
@@ -460,17 +470,13 @@ int synth_batch_phase(const ac_synth_job *jobs, int32_t num_jobs, const ac_synth
     }
     cell_prefix[num_jobs] = cells;
     sample_prefix[num_jobs] = samples;
-    // Filter units, longest job first (stable), six per job, padded to whole warps.
-    std::vector<int32_t> order(static_cast<size_t>(num_jobs));
+    // Filter order, longest job first (stable), padded to whole blocks.
     for (int32_t j = 0; j < num_jobs; ++j) order[j] = j;
-    std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
+    std::stable_sort(order, order + num_jobs, [&](int32_t a, int32_t b) {
         return static_cast<int64_t>(jobs[a].num_bins) * jobs[a].samples_per_bin >
                static_cast<int64_t>(jobs[b].num_bins) * jobs[b].samples_per_bin;
     });
-    int32_t u = 0;
-    for (const int32_t j : order)
-        for (int band = 0; band < 6; ++band) units[u++] = (j << 3) | band;
-    for (; u < l.num_units; ++u) units[u] = -1;
+    for (int32_t u = num_jobs; u < l.num_slots; ++u) order[u] = -1;
 
     AC_CUDA_TRY(cudaMemcpyAsync(ws, host, l.table_end, cudaMemcpyHostToDevice, stream));
     if (!host_staging) AC_CUDA_TRY(cudaStreamSynchronize(stream));  // pageable source must stay alive
@@ -484,11 +490,7 @@ int synth_batch_phase(const ac_synth_job *jobs, int32_t num_jobs, const ac_synth
     const int raw_grid = static_cast<int>(std::min<int64_t>((samples + 255) / 256, 65536));
     ac::synth_batch_raw_kernel<<<raw_grid, 256, 0, stream>>>(d_jobs, d_samples, num_jobs, amps, air, raw);
     AC_CUDA_TRY(cudaGetLastError());
-    if (filter_phase) {
-        ac::synth_batch_filter_kernel<<<l.num_units / 4, 32, 0, stream>>>(d_jobs, d_units, l.num_units, *config, raw);
-        AC_CUDA_TRY(cudaGetLastError());
-    }
-    return AC_OK;
+    return filter_phase ? ac::launch_batch_filter(d_jobs, d_order, num_jobs, *config, raw, stream) : AC_OK;
 }
 
 }  // namespace
