@@ -7,31 +7,31 @@
 // operation order.  The network is sequential in time, but its feedback runs
 // through delay lines of at least AC_FDN_MIN_DELAY samples, so nothing a
 // sample computes is needed by the next hundred samples except each biquad's
-// own state.  A biquad's state recursion ((S - a1*y1) - a2*y2) is three
-// dependent float64 operations per sample; a sample needs 96 absorptive
-// sections, and one warp issuing three of them per lane is bound by the
-// float64 issue rate, so the sections are spread one per lane.  One
-// 192-thread block renders one impulse response:
+// own state.  What bounds it is that state, ((S - a1*y1) - a2*y2): three
+// dependent float64 operations of 8.3 cycles per sample (25 cycles).  One
+// 256-thread block renders one impulse response in steps of S samples, a job
+// per warp, one recursion warp per scheduler:
 //
-//   warps 0-3 (the lines): lane 6j + b of warp w runs absorptive section
-//     (band) b of line 4w + j, kLineSkew steps behind band b - 1, whose
-//     output reaches it by a shuffle; the input part of each biquad is
-//     computed a step ahead, so only its three-operation recursion is on the
-//     per-sample path.  Lanes 24-31 idle.  Band 5 of sample m runs at step m + kLineLag and is
-//     stored to a shared ring.  Each warp fetches its four delay lines one
-//     32-sample block ahead by cp.async.
-//   warp 4 (the mix): one block behind, lane i takes sample i of the block
-//     from the ring and, in registers, sums its sixteen line outputs in line
-//     order, runs the Hadamard butterfly and writes the sixteen delay lines
-//     (global memory, L2-resident; coalesced per line), and runs the four
-//     all-pass stages (their delays exceed 32, so a block's samples are
-//     independent).
-//   warp 5 (the tone): two blocks behind, the six tone sections as a
-//     systolic chain over lanes 0-5, kToneSkew steps apart.
+//   warps 0-2: the 96 absorptive sections, one per lane, sixteen lines of two
+//       bands per warp, each S samples in a row from one column of shared
+//       memory to the next (Biquad::run);
+//   warp 3: the six sections of the output cascade, a lane each;
+//   warp 4: the Hadamard mix and the delay lines' new samples (global memory,
+//       L2-resident, coalesced per line), lane i taking sample i of the step;
+//   warp 5: the sum of the line outputs and the four all-pass stages (their
+//       delays are S or more, so a step's samples are independent);
+//   warp 6: the delay lines' next samples;
+//   warp 7: the output.
 //
-// The six warps meet at one named barrier per block.  A delay-line value
-// written by the mix warp is visible to the line warps two barriers later,
-// which is why the delays must be at least 128 samples (see check_fdn).
+// Band b + 1 runs one step behind band b, so a sample's feedback is written in
+// the sixth step after its first section's, and the step size is picked to fit
+// the shortest delay (fdn_step).  8 impulses of 121,952 samples (48 kHz, S = 64):
+// 2.47 ms (43 cycles per sample) against 4.3 ms (76) with shuffles between the
+// bands of a line in every sample and a barrier every 32; 256 of 30,000 samples
+// (16 kHz, S = 32, two blocks per SM) 1.35 ms against 1.94, 1,184 of them 6.1
+// against 8.1, where the shared-memory pipe is 66 % busy.  Input parts on warps of their own, as in
+// band_filter.cuh, took 44 cycles: they double the shared-memory traffic, which
+// with 96 sections is then what bounds the step.
 //
 // ac_late_tail restates the rest of _render_parametric_fdn_late_reverb
 // (:2588-2640): bandlimit_band_signals of the impulse (the crossover filter
@@ -43,7 +43,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <mutex>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -55,24 +54,9 @@ namespace ac {
 namespace {
 
 constexpr int kLines = AC_FDN_LINES;
-constexpr int kBlk = 32;                   // samples per block
-constexpr int kLineSkew = 2;               // steps between consecutive absorptive sections of a line
-constexpr int kLineWarps = 4;              // line warps, four lines each
-constexpr int kLinesPerWarp = kLines / kLineWarps;
-constexpr int kLineLag = 5 * kLineSkew;        // band 5 of sample m runs at step m + kLineLag
-constexpr int kRing = 4 * kBlk;            // samples of line outputs kept for the output warp
-constexpr int kRowStride = kLines + 1;     // doubles per ring row: column reads without bank conflicts
-constexpr int kToneSkew = 2;               // steps between consecutive tone sections
-constexpr int kToneLag = 5 * kToneSkew;    // tone section 5 finishes sample g - kToneLag at step g
-constexpr int kStageRow = kLines + 1;      // staged inputs: one padded row of 16 lines per sample
-constexpr int kStageBlock = kBlk * kStageRow;
-constexpr int kStageDoubles = 2 * kStageBlock;
-constexpr int kFixedSmem = (kStageDoubles + kRing * kRowStride + 3 * kBlk) * static_cast<int>(sizeof(double));
-constexpr int kFdnThreads = 32 * (kLineWarps + 2);
-// Warp 1 writes the delay-line values of sample block b between barriers b+1
-// and b+2; warp 0's prefetch after barrier j-1 reads samples up to 32j + 63,
-// whose delayed sources must lie in blocks <= j - 3: delays of 128 or more.
-static_assert(AC_FDN_MIN_DELAY >= 4 * kBlk, "a prefetched delay-line value must be visible to warp 0");
+constexpr int kBandSections = 6;
+constexpr int kTonePitch = kBandSections + 1;
+constexpr int kMinAllpass = 32;   // all-pass delays must exceed this
 
 inline size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 
@@ -89,11 +73,32 @@ struct FdnJobDev {
     int64_t pool;                   // offset of this job's delay lines in the workspace pool (doubles)
 };
 
-// y = b0*x + b1*x1 + b2*x2 - a1*y1 - a2*y2, left to right, all in float64
-// (the absorptive and tone sections of steam_rt.py:2261-2275 / :2312-2325).
-// feed() is the input part ((b0*x + b1*x1) + b2*x2), which does not depend on
-// y and is computed one sample ahead; step() is the recursion
-// (v - a1*y1) - a2*y2.  Same operations in the same order as run().
+// A delay line as the loader and the mix see it: its offset in the pool, its length, and the position of the first
+// sample of their next step.
+struct FdnLine {
+    int start, delay, pos, pad;
+};
+
+// Steps of S samples.  Each buffer is doubled: what one warp writes in a step others read in the next.
+template <int S>
+struct FdnSmem {
+    // columns: the delay lines' samples, then the outputs of bands 0 .. 5, sixteen lines each (an odd pitch: the mix
+    // reads rows per lane)
+    static constexpr int kPitch = kLines * (1 + kBandSections) + 1;
+    double y[2][S][kPitch];
+    double t[2][S][kTonePitch];            // [0]: the output of the all-passes, [s + 1]: of tone section s
+    FdnLine load_line[kLines], mix_line[kLines];
+};
+
+constexpr int kFdnThreads = 256;
+// What a sample computes reaches the delay lines in the sixth step after its first section's, and the lines are read
+// two steps ahead: the pipeline needs delays of at least kFdnLatency * S samples.
+constexpr int kFdnLatency = 9;
+
+// One absorptive or tone section (steam_rt.py:2261-2275, :2312-2325) of one lane, in float64:
+//     y0 = b0*x0 + b1*x1 + b2*x2 - a1*y1 - a2*y2, left to right.
+// The input part ((b0*x0 + b1*x1) + b2*x2) does not depend on y and is formed four samples ahead, so its products fill
+// the gaps of the recursion (v - a1*y1) - a2*y2.
 struct Biquad {
     double b0, b1, b2, a1, a2, x1, x2, y1, y2;
 
@@ -110,223 +115,234 @@ struct Biquad {
     }
 
     __device__ __forceinline__ double step(double v) {
-        const double y = v - a1 * y1 - a2 * y2;
+        const double y0 = v - a1 * y1 - a2 * y2;
         y2 = y1;
-        y1 = y;
-        return y;
+        y1 = y0;
+        return y0;
+    }
+
+    // S samples from column xp to column yp of rows kPitch apart.
+    template <int S, int kPitch>
+    __device__ __forceinline__ void run(const double *xp, double *yp) {
+        constexpr int kAhead = 4;
+        static_assert(S % kAhead == 0, "whole groups");
+        double v[kAhead], x[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) x[u] = xp[u * kPitch];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) v[u] = feed(x[u]);
+        // not unrolled whole: the warps run different code, and with straight-line code for a step of 64 samples a full
+        // GPU (148 impulses) fell from 47 to 77-112 cycles per sample waiting for instructions
+#pragma unroll 4
+        for (int base = kAhead; base < S; base += kAhead) {
+            double vn[kAhead];
+            xp += kAhead * kPitch;
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) x[u] = xp[u * kPitch];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                yp[u * kPitch] = step(v[u]);
+                vn[u] = feed(x[u]);
+            }
+            yp += kAhead * kPitch;
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) v[u] = vn[u];
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) yp[u * kPitch] = step(v[u]);
     }
 };
 
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// The six warps of a block meet here once per sample block.
-__device__ __forceinline__ void block_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kFdnThreads) : "memory"); }
-
-// Block k's delay-line inputs for lines first .. first + 3: lane i fetches
-// sample 32k + i of each into row i of the stage; advance the positions by
-// one block.
-__device__ __forceinline__ void prefetch_block(const double *lines, const int *line_start, const int *delays,
-                                               int first, int *pos, double *stage, int lane) {
-#pragma unroll
-    for (int j = 0; j < kLinesPerWarp; ++j) {
-        const int l = first + j;
-        cp_async8(stage + lane * kStageRow + l, lines + line_start[l] + pos[j]);
-        const int p = pos[j] + kBlk;
-        pos[j] = p >= delays[l] ? p - delays[l] : p;
-    }
-    cp_async_commit();
-}
-
-__device__ void fdn_lines(const FdnJobDev &job, const double *lines, double *stage, double *rows, const int *s_start,
-                          const int *s_delay, int iterations) {
-    const unsigned full = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31;
-    const int first = (threadIdx.x >> 5) * kLinesPerWarp;
-    const bool valid = lane < 6 * kLinesPerWarp;
-    const int line = first + (valid ? lane / 6 : 0);
-    const int band = valid ? lane % 6 : 0;
-    Biquad sec;
-    sec.load(job.absorptive[line][band]);
-    if (!valid) sec.b0 = sec.b1 = sec.b2 = sec.a1 = sec.a2 = 0.0;
-    const bool stores = valid && band == 5;
-    int pos[kLinesPerWarp];
-#pragma unroll
-    for (int j = 0; j < kLinesPerWarp; ++j) pos[j] = lane;  // every delay exceeds 32
-    // band b works on sample n - kLineSkew * b at step n; its input is band b - 1's output of step
-    // n - kLineSkew, which arrives by a shuffle issued at step n - kLineSkew and is fed (the input part
-    // of the biquad) one step ahead, at step n - 1
-    static_assert(kLineSkew == 2, "the shuffle is consumed one step after it is issued");
-    double received = 0.0;   // band b - 1's output of the previous step
-    double carry = 0.0;      // band b - 1's input for the first step of the next block
-    double v = 0.0;          // input part for the current step
-    prefetch_block(lines, s_start, s_delay, first, pos, stage, lane);
-    for (int k = 0; k < iterations; ++k) {
-        prefetch_block(lines, s_start, s_delay, first, pos, stage + ((k + 1) & 1) * kStageBlock, lane);
-        cp_async_wait<1>();
-        __syncwarp();
-        const double *in = stage + (k & 1) * kStageBlock + line;
-        v = sec.feed(band == 0 ? in[0] : carry);
-        const int m0 = k * kBlk - kLineLag;
-        // fully unrolled, so that band 0's staged reads are issued well ahead of their use
-#pragma unroll
-        for (int t = 0; t < kBlk; ++t) {
-            const double y = sec.step(v);                      // the only chain carried between steps
-            const double next_in = band == 0 ? in[((t + 1) & (kBlk - 1)) * kStageRow] : received;
-            received = __shfl_up_sync(full, y, 1);
-            if (t + 1 < kBlk) v = sec.feed(next_in);          // the next block's first input is fed after its fetch
-            else carry = next_in;
-            // band 5 of sample m0 + t; the ring slots written while m0 + t < 0 (zeros) are
-            // rewritten with their real samples before the mix warp reads them
-            if (stores) rows[((m0 + t) & (kRing - 1)) * kRowStride + line] = y;
-        }
-        __syncwarp();
-        block_barrier();
-    }
-    cp_async_wait<0>();
-}
-
-__device__ void fdn_mix(const FdnJobDev &job, double *lines, const double *rows, double *tone_in, double *ap,
-                        const int *s_start, const int *s_delay, int blocks, int iterations) {
-    const int lane = threadIdx.x & 31;
-    int apos[AC_FDN_ALLPASS];
-#pragma unroll
-    for (int s = 0; s < AC_FDN_ALLPASS; ++s) apos[s] = 0;
-    int wpos[kLines];   // delay-line position of this lane's sample in the current block
-#pragma unroll
-    for (int l = 0; l < kLines; ++l) wpos[l] = lane;
-    for (int k = 0; k < iterations; ++k) {
-        block_barrier();
-        if (k == 0 || k > blocks) continue;
-        const int base = (k - 1) * kBlk;  // samples base .. base + 31 are complete in the ring
-        const int m = base + lane;
-        const double *row = rows + (m & (kRing - 1)) * kRowStride;
-        double d[kLines];
-#pragma unroll
-        for (int l = 0; l < kLines; ++l) d[l] = row[l];
-        // output: the line outputs summed in line order, over the line count (steam_rt.py:2297-2300)
-        double v = 0.0;
-#pragma unroll
-        for (int l = 0; l < kLines; ++l) v += d[l];
-        v /= static_cast<double>(kLines);
-        // feedback: unnormalised Hadamard butterfly, strides 1, 2, 4, 8, written back with gain 0.25
-        // and the unit impulse at sample 0 (steam_rt.py:2279-2295)
-#pragma unroll
-        for (int stride = 1; stride < kLines; stride *= 2)
-#pragma unroll
-            for (int a = 0; a < kLines; ++a)
-                if ((a & stride) == 0) {
-                    const double first = d[a], second = d[a + stride];
-                    d[a] = first + second;
-                    d[a + stride] = first - second;
-                }
-        const double injection = m == 0 ? 1.0 : 0.0;
-#pragma unroll
-        for (int l = 0; l < kLines; ++l) {
-            lines[s_start[l] + wpos[l]] = injection + 0.25 * d[l];
-            const int p = wpos[l] + kBlk;
-            wpos[l] = p >= s_delay[l] ? p - s_delay[l] : p;
-        }
-#pragma unroll
-        for (int s = 0; s < AC_FDN_ALLPASS; ++s) {
-            const int D = job.allpass[s];
-            double *ring = ap + job.allpass_start[s];
-            int idx = apos[s] + lane;
-            idx = idx >= D ? idx - D : idx;
-            const double previous = ring[idx];
-            const double internal = v + 0.5 * previous;
-            ring[idx] = internal;
-            v = previous - 0.5 * internal;
-            const int p = apos[s] + kBlk;
-            apos[s] = p >= D ? p - D : p;
-        }
-        tone_in[((k - 1) & 1) * kBlk + lane] = v;
-    }
-}
-
-__device__ void fdn_tone(const FdnJobDev &job, const double *tone_in, double *tone_out, int blocks, int iterations,
-                         int total) {
-    const unsigned full = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31;
-    Biquad tone;
-    tone.load(job.tone[lane < 6 ? lane : 0]);
-    if (lane >= 6) tone.b0 = tone.b1 = tone.b2 = tone.a1 = tone.a2 = 0.0;
-    static_assert(kToneSkew == 2, "the shuffle is consumed one step after it is issued");
-    // Tone section `lane` works on sample g - kToneSkew * lane at step g; its input is the previous
-    // section's output of step g - kToneSkew, fed one step ahead like the line sections.
-    double received = 0.0, carry = 0.0, v = 0.0;
-    const int preroll = job.preroll;
-    double *out = job.out;
-    // section 5 stages its output of step base + t in tone_out[t]; the warp writes the block out after it
-    const bool last_section = lane == 5;
-    auto flush = [&](int base, int count) {
-        __syncwarp();
-        const int m = base + lane - kToneLag;
-        if (lane < count && m >= preroll && m < total) out[m - preroll] = tone_out[lane];
-        __syncwarp();
-    };
-    for (int k = 0; k < iterations; ++k) {
-        block_barrier();
-        if (k < 2 || k > blocks + 1) continue;
-        const int base = (k - 2) * kBlk;
-        const double *in = tone_in + ((k - 2) & 1) * kBlk;
-        v = tone.feed(lane == 0 ? in[0] : carry);
-#pragma unroll
-        for (int t = 0; t < kBlk; ++t) {
-            const double y = tone.step(v);
-            const double next_in = lane == 0 ? in[(t + 1) & (kBlk - 1)] : received;
-            received = __shfl_up_sync(full, y, 1);
-            if (t + 1 < kBlk) v = tone.feed(next_in);
-            else carry = next_in;
-            if (last_section) tone_out[t] = y;
-        }
-        flush(base, kBlk);
-    }
-    // drain: inputs past the last sample are zero
-    v = tone.feed(lane == 0 ? 0.0 : carry);
-    for (int t = 0; t < kToneLag; ++t) {
-        const double y = tone.step(v);
-        const double next_in = lane == 0 ? 0.0 : received;
-        received = __shfl_up_sync(full, y, 1);
-        v = tone.feed(next_in);
-        if (last_section) tone_out[t] = y;
-    }
-    flush(blocks * kBlk, kToneLag);
-}
-
-__global__ void __launch_bounds__(kFdnThreads) fdn_kernel(const FdnJobDev *jobs, double *pool) {
-    extern __shared__ __align__(16) double smem[];
-    double *stage = smem;
-    double *rows = stage + kStageDoubles;
-    double *tone_in = rows + kRing * kRowStride;
-    double *tone_out = tone_in + 2 * kBlk;
-    double *ap = tone_out + kBlk;
-    __shared__ int s_start[kLines], s_delay[kLines];
+template <int S>
+__global__ void __launch_bounds__(kFdnThreads, 2) fdn_kernel(const FdnJobDev *jobs, double *pool) {
+    constexpr int kPitch = FdnSmem<S>::kPitch, kPasses = (S + 31) / 32;
+    extern __shared__ __align__(16) unsigned char fdn_smem_raw[];
+    FdnSmem<S> &m = *reinterpret_cast<FdnSmem<S> *>(fdn_smem_raw);
+    double *ap = reinterpret_cast<double *>(fdn_smem_raw + sizeof(FdnSmem<S>));
     const FdnJobDev &job = jobs[blockIdx.x];
+    double *lines = pool + job.pool;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int total = job.preroll + job.num_samples;
-    const int blocks = (total + kBlk - 1) / kBlk;
-    // every warp passes the block barrier `iterations` times: the lines finish block b in iteration b + 1,
-    // the mix takes it in iteration b + 1 and the tone in iteration b + 2
-    const int iterations = blocks + 2;
+    const int blocks = (total + S - 1) / S;
+    const int steps = blocks + 13;   // a step's outputs are written 13 steps after its first section
     const int ap_total = job.allpass_start[AC_FDN_ALLPASS - 1] + job.allpass[AC_FDN_ALLPASS - 1];
-    for (int i = threadIdx.x; i < ap_total; i += blockDim.x) ap[i] = 0.0;
+    for (int i = threadIdx.x; i < ap_total; i += kFdnThreads) ap[i] = 0.0;
     if (threadIdx.x < kLines) {
-        s_start[threadIdx.x] = job.line_start[threadIdx.x];
-        s_delay[threadIdx.x] = job.delays[threadIdx.x];
+        const FdnLine line{job.line_start[threadIdx.x], job.delays[threadIdx.x], 0, 0};
+        m.load_line[threadIdx.x] = m.mix_line[threadIdx.x] = line;
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5;
-    if (warp < kLineWarps)
-        fdn_lines(job, pool + job.pool, stage, rows, s_start, s_delay, iterations);
-    else if (warp == kLineWarps)
-        fdn_mix(job, pool + job.pool, rows, tone_in, ap, s_start, s_delay, blocks, iterations);
-    else
-        fdn_tone(job, tone_in, tone_out, blocks, iterations, total);
+    // all warps meet here once per step
+    auto barrier = [] {
+        __syncwarp();
+        asm volatile("bar.sync 1, %0;" ::"n"(kFdnThreads) : "memory");
+    };
+    // lane's sample (pass h) of line l in the step that `table` stands at; advance() moves it one step on
+    auto offset_of = [&](const FdnLine *table, int l, int h) {
+        const FdnLine line = table[l];
+        const int p = line.pos + 32 * h + lane;
+        return line.start + (p >= line.delay ? p - line.delay : p);
+    };
+    auto advance = [&](FdnLine *table) {
+        __syncwarp();
+        if (lane < kLines) {
+            const int p = table[lane].pos + S;
+            table[lane].pos = p >= table[lane].delay ? p - table[lane].delay : p;
+        }
+        __syncwarp();
+    };
+
+    if (warp < 3) {
+        // bands 2 * warp and 2 * warp + 1 of the sixteen lines; band b works on step i - b
+        const int band = 2 * warp + (lane >> 4), column = band * kLines + (lane & 15);
+        Biquad section;
+        section.load(job.absorptive[lane & 15][band]);
+        barrier();
+        for (int i = 0; i < steps; ++i) {
+            const int k = i - band;
+            if (k >= 0 && k < blocks)
+                section.run<S, kPitch>(&m.y[k & 1][0][column], &m.y[k & 1][0][column + kLines]);
+            barrier();
+        }
+    } else if (warp == 3) {
+        // tone section `lane`, on step i - 7 - lane
+        Biquad section;
+        section.load(job.tone[lane < kBandSections ? lane : 0]);
+        barrier();
+        for (int i = 0; i < steps; ++i) {
+            const int k = i - 7 - lane;
+            if (lane < kBandSections && k >= 0 && k < blocks)
+                section.run<S, kTonePitch>(&m.t[k & 1][0][lane], &m.t[k & 1][0][lane + 1]);
+            barrier();
+        }
+    } else if (warp == 4) {
+        // the feedback: a sample per lane, an unnormalised Hadamard butterfly of the line outputs, strides 1, 2, 4, 8,
+        // written back with gain 0.25 and the unit impulse at sample 0 (steam_rt.py:2279-2295)
+        barrier();
+        for (int i = 0; i < steps; ++i) {
+            const int k = i - kBandSections;
+            if (k >= 0 && k < blocks) {
+#pragma unroll 1
+                for (int h = 0; h < kPasses; ++h) {
+                    const int r = 32 * h + lane;
+                    if (r < S) {
+                        int offset[kLines];   // all addresses before the first store, which a later load would wait for
+#pragma unroll
+                        for (int l = 0; l < kLines; ++l) offset[l] = offset_of(m.mix_line, l, h);
+                        const double *row = &m.y[k & 1][r][kBandSections * kLines];
+                        double d[kLines];
+#pragma unroll
+                        for (int l = 0; l < kLines; ++l) d[l] = row[l];
+#pragma unroll
+                        for (int stride = 1; stride < kLines; stride *= 2)
+#pragma unroll
+                            for (int a = 0; a < kLines; ++a)
+                                if ((a & stride) == 0) {
+                                    const double one = d[a], two = d[a + stride];
+                                    d[a] = one + two;
+                                    d[a + stride] = one - two;
+                                }
+                        const double injection = k == 0 && r == 0 ? 1.0 : 0.0;
+#pragma unroll
+                        for (int l = 0; l < kLines; ++l) lines[offset[l]] = injection + 0.25 * d[l];
+                    }
+                }
+                advance(m.mix_line);
+            }
+            barrier();
+        }
+    } else if (warp == 5) {
+        // the output of the network, a sample per lane: the line outputs summed in line order, over the line count
+        // (steam_rt.py:2297-2300), through the four all-passes
+        int apos[AC_FDN_ALLPASS], ap_delay[AC_FDN_ALLPASS], ap_start[AC_FDN_ALLPASS];
+#pragma unroll
+        for (int s = 0; s < AC_FDN_ALLPASS; ++s) {
+            ap_delay[s] = job.allpass[s];
+            ap_start[s] = job.allpass_start[s];
+            apos[s] = 0;
+        }
+        barrier();
+        for (int i = 0; i < steps; ++i) {
+            const int k = i - kBandSections;
+            if (k >= 0 && k < blocks) {
+#pragma unroll 1
+                for (int h = 0; h < kPasses; ++h) {
+                    const int r = 32 * h + lane;
+                    if (r < S) {
+                        const double *row = &m.y[k & 1][r][kBandSections * kLines];
+                        double d[kLines], previous[AC_FDN_ALLPASS];
+                        int cell[AC_FDN_ALLPASS];
+#pragma unroll
+                        for (int l = 0; l < kLines; ++l) d[l] = row[l];
+#pragma unroll
+                        for (int s = 0; s < AC_FDN_ALLPASS; ++s) {
+                            const int p = apos[s] + r;
+                            cell[s] = ap_start[s] + (p >= ap_delay[s] ? p - ap_delay[s] : p);
+                            previous[s] = ap[cell[s]];
+                        }
+                        double v = 0.0;
+#pragma unroll
+                        for (int l = 0; l < kLines; ++l) v += d[l];
+                        v /= static_cast<double>(kLines);
+#pragma unroll
+                        for (int s = 0; s < AC_FDN_ALLPASS; ++s) {
+                            const double internal = v + 0.5 * previous[s];
+                            ap[cell[s]] = internal;
+                            v = previous[s] - 0.5 * internal;
+                        }
+                        m.t[k & 1][r][0] = v;
+                    }
+                }
+#pragma unroll
+                for (int s = 0; s < AC_FDN_ALLPASS; ++s) {
+                    const int p = apos[s] + S;
+                    apos[s] = p >= ap_delay[s] ? p - ap_delay[s] : p;
+                }
+            }
+            barrier();
+        }
+    } else if (warp == 6) {
+        // the delay lines' samples, a sample per lane, read two steps ahead (around L1: the mix writes them) and
+        // stored to the next step's buffer; sample n of a line is at n mod delay
+        double x[kPasses][kLines];
+        auto fetch = [&] {
+#pragma unroll
+            for (int h = 0; h < kPasses; ++h)
+#pragma unroll
+                for (int l = 0; l < kLines; ++l)
+                    x[h][l] = 32 * h + lane < S ? __ldcg(lines + offset_of(m.load_line, l, h)) : 0.0;
+            advance(m.load_line);
+        };
+        auto store = [&](int k) {
+#pragma unroll
+            for (int h = 0; h < kPasses; ++h)
+#pragma unroll
+                for (int l = 0; l < kLines; ++l)
+                    if (32 * h + lane < S) m.y[k & 1][32 * h + lane][l] = x[h][l];
+        };
+        fetch();
+        store(0);
+        fetch();
+        barrier();
+        for (int i = 0; i < steps; ++i) {
+            store(i + 1);   // (past the last block: samples that nothing reads)
+            fetch();        // of step i + 2
+            barrier();
+        }
+    } else {
+        const int preroll = job.preroll;
+        double *out = job.out;
+        barrier();
+        for (int i = 0; i < steps; ++i) {
+            const int k = i - 13;
+#pragma unroll
+            for (int h = 0; h < kPasses; ++h) {
+                const int r = 32 * h + lane, n = k * S + r;
+                if (r < S && k >= 0 && n >= preroll && n < total) out[n - preroll] = m.t[k & 1][r][kBandSections];
+            }
+            barrier();
+        }
+    }
 }
 
 // ---- the hybrid tail ------------------------------------------------------
@@ -527,12 +543,14 @@ struct FdnLayout {
     size_t jobs, pool, total;
     int64_t pool_doubles;
     int max_allpass_doubles;
+    int min_delay, min_allpass;
 };
 
 int check_fdn(const ac_fdn_job *jobs, int32_t num_jobs, bool need_buffers, FdnLayout *out) {
     if (num_jobs < 0 || (num_jobs > 0 && !jobs)) return fail(AC_ERR_INVALID, "fdn: null argument");
     if (num_jobs > (1 << 24)) return fail(AC_ERR_CAPACITY, "fdn batch of %d jobs is too large", num_jobs);
     FdnLayout l{};
+    l.min_delay = l.min_allpass = 1 << 30;
     for (int32_t j = 0; j < num_jobs; ++j) {
         const ac_fdn_job &job = jobs[j];
         int64_t lines = 0;
@@ -541,14 +559,16 @@ int check_fdn(const ac_fdn_job *jobs, int32_t num_jobs, bool need_buffers, FdnLa
                 return fail(AC_ERR_INVALID, "fdn job %d: delay %d of line %d outside [%d, 2^26]", j, job.delays[i], i,
                             AC_FDN_MIN_DELAY);
             lines += job.delays[i];
+            l.min_delay = std::min(l.min_delay, job.delays[i]);
         }
         if (lines > 0x7FFFFFFF) return fail(AC_ERR_CAPACITY, "fdn job %d: delay lines too long", j);
         int ap = 0;
         for (int s = 0; s < AC_FDN_ALLPASS; ++s) {
-            if (job.allpass_delays[s] <= kBlk || job.allpass_delays[s] > AC_FDN_MAX_ALLPASS)
+            if (job.allpass_delays[s] <= kMinAllpass || job.allpass_delays[s] > AC_FDN_MAX_ALLPASS)
                 return fail(AC_ERR_INVALID, "fdn job %d: all-pass delay %d outside [%d, %d]", j, job.allpass_delays[s],
-                            kBlk + 1, AC_FDN_MAX_ALLPASS);
+                            kMinAllpass + 1, AC_FDN_MAX_ALLPASS);
             ap += job.allpass_delays[s];
+            l.min_allpass = std::min(l.min_allpass, job.allpass_delays[s]);
         }
         if (job.num_samples < 0 || job.preroll < 0 ||
             static_cast<int64_t>(job.num_samples) + job.preroll > (int64_t{1} << 30))
@@ -570,18 +590,33 @@ int check_fdn(const ac_fdn_job *jobs, int32_t num_jobs, bool need_buffers, FdnLa
     return AC_OK;
 }
 
-std::mutex g_smem_mutex;
-int g_smem_set[64] = {0};
+constexpr int kMaxSmem = 227 * 1024;
 
-// Opt the FDN kernel into the dynamic shared memory it needs on this device.
-int ensure_fdn_smem(int bytes) {
-    int dev = 0;
-    AC_CUDA_TRY(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lock(g_smem_mutex);
-    const int slot = dev & 63;
-    if (g_smem_set[slot] >= bytes) return AC_OK;
-    AC_CUDA_TRY(cudaFuncSetAttribute(fdn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    g_smem_set[slot] = bytes;
+// The step size of a launch: the largest whose pipeline fits the batch's shortest delay (kFdnLatency steps), whose
+// all-pass samples are independent within a step and whose buffers fit shared memory.  A larger step has fewer barriers
+// per sample, but a step of 64 takes a whole SM (135 KB), so beyond one impulse per SM a step of 32, two blocks per SM,
+// is faster (296 impulses of 48 kHz: 72 cycles per sample against two waves of 47).  A step of 40 would fit the designs
+// of 16 kHz, but its mix takes two passes of 32 lanes and it is no faster (54 cycles against 47).  The reference's designs have delays of at least 841 samples from 32 kHz up, 361 at 16 kHz and 289 from
+// 7 kHz; a step of 8 meets every accepted delay.
+int fdn_step(const FdnLayout &l, int num_jobs, int sms) {
+    const size_t ap = static_cast<size_t>(l.max_allpass_doubles) * sizeof(double);
+    auto fits = [&](int step, size_t smem) {
+        return kFdnLatency * step <= l.min_delay && step <= l.min_allpass && smem + ap <= kMaxSmem;
+    };
+    if (num_jobs <= sms && fits(64, sizeof(FdnSmem<64>))) return 64;
+    if (fits(32, sizeof(FdnSmem<32>))) return 32;
+    return 8;
+}
+static_assert(kFdnLatency * 8 <= AC_FDN_MIN_DELAY && 8 <= kMinAllpass, "a step of 8 meets every accepted design");
+static_assert(sizeof(FdnSmem<8>) + AC_FDN_ALLPASS * AC_FDN_MAX_ALLPASS * sizeof(double) <= kMaxSmem, "and fits");
+
+template <int S>
+int launch_fdn(const FdnJobDev *jobs, int num_jobs, double *pool, int max_allpass_doubles, cudaStream_t stream) {
+    const size_t smem = sizeof(FdnSmem<S>) + static_cast<size_t>(max_allpass_doubles) * sizeof(double);
+    // always the same limit: a concurrent call with other all-pass lengths must not lower it
+    AC_CUDA_TRY(cudaFuncSetAttribute(fdn_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
+    fdn_kernel<S><<<num_jobs, kFdnThreads, smem, stream>>>(jobs, pool);
+    AC_CUDA_TRY(cudaGetLastError());
     return AC_OK;
 }
 
@@ -683,13 +718,16 @@ extern "C" int ac_fdn_impulse(const ac_fdn_job *jobs, int32_t num_jobs, void *wo
     AC_CUDA_TRY(cudaMemcpyAsync(ws + l.jobs, host, table_bytes, cudaMemcpyHostToDevice, stream));
     if (!host_staging) AC_CUDA_TRY(cudaStreamSynchronize(stream));  // pageable source must stay alive
     AC_CUDA_TRY(cudaMemsetAsync(ws + l.pool, 0, static_cast<size_t>(l.pool_doubles) * sizeof(double), stream));
-    const int smem = ac::kFixedSmem + l.max_allpass_doubles * static_cast<int>(sizeof(double));
-    const int prc = ac::ensure_fdn_smem(smem);
-    if (prc != AC_OK) return prc;
-    ac::fdn_kernel<<<num_jobs, ac::kFdnThreads, smem, stream>>>(reinterpret_cast<const ac::FdnJobDev *>(ws + l.jobs),
-                                                   reinterpret_cast<double *>(ws + l.pool));
-    AC_CUDA_TRY(cudaGetLastError());
-    return AC_OK;
+    int device = 0, sms = 0;
+    AC_CUDA_TRY(cudaGetDevice(&device));
+    AC_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const ac::FdnJobDev *d_jobs = reinterpret_cast<const ac::FdnJobDev *>(ws + l.jobs);
+    double *lines = reinterpret_cast<double *>(ws + l.pool);
+    switch (ac::fdn_step(l, num_jobs, sms)) {
+        case 64: return ac::launch_fdn<64>(d_jobs, num_jobs, lines, l.max_allpass_doubles, stream);
+        case 32: return ac::launch_fdn<32>(d_jobs, num_jobs, lines, l.max_allpass_doubles, stream);
+        default: return ac::launch_fdn<8>(d_jobs, num_jobs, lines, l.max_allpass_doubles, stream);
+    }
 }
 
 extern "C" int ac_late_tail_workspace_size(const ac_late_tail_job *jobs, int32_t num_jobs,
