@@ -161,6 +161,8 @@ class Builder {
         return f;
     }
 
+    // Both children's bounds, {lo.x, hi.x, lo.y, hi.y} each, {lo.z, hi.z} each, references: what the four-wide collapse
+    // reads; centre_form turns it into the binary layout.
     void write_node(int64_t node, const Box &l, int32_t lref, const Box &r, int32_t rref) {
         float *q = out_->nodes.data() + 16 * node;
         q[0] = down(l.lo[0]); q[1] = up(l.hi[0]); q[2] = down(l.lo[1]); q[3] = up(l.hi[1]);
@@ -248,6 +250,29 @@ class Collapser {
     const std::vector<float> &bin_;
 };
 
+// The binary layout's final form (fast_bvh.h): each child's box as centre and half extent, the extent rounded up so
+// that the box still covers its float32 bounds.
+void centre_form(std::vector<float> &nodes) {
+    for (size_t n = 0; n < nodes.size(); n += 16) {
+        float q[16];
+        std::copy(nodes.begin() + n, nodes.begin() + n + 16, q);
+        for (int side = 0; side < 2; ++side) {
+            float *out = nodes.data() + n + 8 * side;
+            for (int a = 0; a < 3; ++a) {
+                const double lo = a < 2 ? q[4 * side + 2 * a] : q[8 + 2 * side], hi = a < 2 ? q[4 * side + 2 * a + 1] : q[9 + 2 * side];
+                const float c = static_cast<float>(0.5 * (lo + hi));
+                const double half = std::max(hi - static_cast<double>(c), static_cast<double>(c) - lo);
+                float e = static_cast<float>(half);
+                if (static_cast<double>(e) < half) e = std::nextafter(e, std::numeric_limits<float>::infinity());
+                out[a] = c;
+                out[4 + a] = e;
+            }
+            out[3] = q[12 + side];   // an int32 bit pattern
+            out[7] = 0.0f;
+        }
+    }
+}
+
 }  // namespace
 
 int build_traversal_bvh(const std::vector<int64_t> &surfaces, const double *lo, const double *hi, int leaf_max,
@@ -292,6 +317,7 @@ int build_traversal_bvh(const std::vector<int64_t> &surfaces, const double *lo, 
             out->stack_need = need + 1;
         }
     }
+    if (out->width == 2) centre_form(out->nodes);
     return AC_OK;
 }
 

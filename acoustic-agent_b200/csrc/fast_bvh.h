@@ -3,13 +3,12 @@
 // A binary BVH over the walls and boxes of a scene, built with the binned
 // surface-area heuristic, laid out for per-lane traversal on the GPU: every
 // inner node stores the boxes of BOTH children (so one node fetch decides the
-// next step), four 16-byte quads per node:
+// next step), 32 bytes per child, read in one load each:
 //
-//   q0 = {c0.lo.x, c0.hi.x, c0.lo.y, c0.hi.y}
-//   q1 = {c1.lo.x, c1.hi.x, c1.lo.y, c1.hi.y}
-//   q2 = {c0.lo.z, c0.hi.z, c1.lo.z, c1.hi.z}
-//   q3 = {ref0, ref1, 0, 0}   (int32 bit patterns)
+//   {centre.x, centre.y, centre.z, ref} {half.x, half.y, half.z, 0}
 //
+// with the reference's int32 bit pattern in `ref` and the half extents rounded
+// up, so that centre +- half covers the padded float32 bounds.
 // A child reference >= 0 is an inner node index; < 0 is a leaf,
 // ~((first << 3) | (count - 1)) over the leaf-ordered surface slots, so a leaf
 // holds 1..8 surfaces.  Node 0 is the root and always an inner node (a scene
