@@ -241,18 +241,21 @@ int pack_and_upload(const ac_scene_desc *d, const ac_bvh &bvh, const FastLists *
             bb[3] = tag_value<T>(static_cast<int>(si) * 4 + AC_KIND_BOX);
         }
         // Polygon edges for the even-odd test: {x_i, y_i, y_j, (x_j - x_i) / (y_j - y_i)} with j the
-        // previous corner (steam_rt.py:4259-4274); an edge the reference skips gets y_j = y_i.
+        // previous corner (steam_rt.py:4259-4274); an edge the reference skips, or whose ends have the same float32 y,
+        // never crosses and is left out.
+        size_t edges = 0;
         for (size_t i = 0; i < C; ++i) {
             const size_t j = (i + C - 1) % C;
             const double xi = d->corners[2 * i], yi = d->corners[2 * i + 1];
             const double xj = d->corners[2 * j], yj = d->corners[2 * j + 1];
-            T *e = host.data() + o.edges + 4 * i;
-            const bool skip = std::fabs(yj - yi) <= 1e-12;
+            if (std::fabs(yj - yi) <= 1e-12 || T(yi) == T(yj)) continue;
+            T *e = host.data() + o.edges + 4 * edges++;
             e[0] = T(xi);
             e[1] = T(yi);
-            e[2] = skip ? T(yi) : T(yj);
-            e[3] = skip ? T(0) : T((xj - xi) / (yj - yi));
+            e[2] = T(yj);
+            e[3] = T((xj - xi) / (yj - yi));
         }
+        s->fast.num_edges = static_cast<int32_t>(edges);
         if (f->use_bvh) {
             std::copy(f->bvh.nodes.begin(), f->bvh.nodes.end(), host.begin() + o.bvh_nodes);
             for (size_t k = 0; k < f->bvh.order.size(); ++k)
@@ -317,7 +320,6 @@ int pack_and_upload(const ac_scene_desc *d, const ac_bvh &bvh, const FastLists *
         s->fast.num_wall_clusters = static_cast<int32_t>(f->wall_clusters.size());
         s->fast.num_polys = static_cast<int32_t>(f->polys.size());
         s->fast.num_box_clusters = static_cast<int32_t>(f->box_clusters.size());
-        s->fast.num_edges = static_cast<int32_t>(C);
         s->num_clusters = static_cast<int64_t>(f->wall_clusters.size() + f->box_clusters.size());
         if (f->use_bvh) {
             // BVH mode: walls and boxes come from the traversal BVH, only polygons stay in the scan;

@@ -55,7 +55,7 @@ struct FastScene {
     const float *box_clusters;   // [NBC][8]
     const float *box_bounds;     // [NB][8]  world AABB {lo.xyz, tag} {hi.xyz, 0}
     const float *boxes;          // [NB][12] box records (trace_kernel.cuh layout)
-    const float *edges;          // [C][4]   {x_i, y_i, y_j (or y_i if skipped), (x_j-x_i)/(y_j-y_i)}
+    const float *edges;          // [E][4]   {x_i, y_i, y_j, (x_j-x_i)/(y_j-y_i)}, edges that a horizontal line can cross
     int32_t num_wall_clusters;
     int32_t num_polys;
     int32_t num_box_clusters;
@@ -474,17 +474,30 @@ __device__ __forceinline__ void scene_scan(const FastScene &fs, const FRay &r, b
             if (pass) take(wall_t(A, B, r), __float_as_int(B.z) >> 2, best_t, best);
         }
     }
-    // Horizontal polygons (floor, ceiling), in lockstep.
+    // Horizontal polygons (floor, ceiling): they share the room's outline, and a ray inside the room reaches the plane of
+    // one of them, so each lane tests its own candidates and the warp walks the outline once for all of them
+    // (instead of once per plane: U room 9.04 -> 8.72 ms, 8-room apartment 7.65 -> 7.44, with the edges that never cross left
+    // out of the outline).
 #pragma unroll 1
-    for (int k = 0; k < fs.num_polys; ++k) {
-        const Quad<float> P = ldq(fs.polys + 4 * k);
-        const float t = (P.x - r.o[2]) * r.inv[2];
-        const int si = __float_as_int(P.y) >> 2;
-        const bool cand = active && !(any_hit && best >= 0) && fabsf(r.d[2]) > 1e-12f && t > 1e-6f &&
-                          (t < best_t || (t == best_t && si < best));
-        if (__any_sync(full, cand)) {
+    for (int first = 0; first < fs.num_polys; first += 32) {
+        unsigned mask = 0u;
+        const bool able = active && !(any_hit && best >= 0) && fabsf(r.d[2]) > 1e-12f;
+        const int count = min(fs.num_polys - first, 32);
+#pragma unroll 1
+        for (int k = 0; k < count; ++k) {
+            const float t = (__ldg(fs.polys + 4 * (first + k)) - r.o[2]) * r.inv[2];
+            if (able && t > 1e-6f && t <= best_t) mask |= 1u << k;
+        }
+#pragma unroll 1
+        while (__any_sync(full, mask != 0u)) {
+            const int k = mask ? __ffs(mask) - 1 : 0;
+            const float2 P = __ldg(reinterpret_cast<const float2 *>(fs.polys + 4 * (first + k)));
+            const float t = (P.x - r.o[2]) * r.inv[2];
+            const int si = __float_as_int(P.y) >> 2;
+            const bool cand = mask != 0u && !(any_hit && best >= 0) && (t < best_t || (t == best_t && si < best));
+            mask &= mask - 1u;
             const float px = r.o[0] + t * r.d[0], py = r.o[1] + t * r.d[1];
-            if (cand && point_in_polygon_fast(px, py, fs.edges, fs.num_edges)) take(t, si, best_t, best);
+            if (point_in_polygon_fast(px, py, fs.edges, fs.num_edges) && cand) take(t, si, best_t, best);
         }
     }
     // Boxes: per-lane candidate masks from world AABBs, then per-lane candidates in lockstep.
