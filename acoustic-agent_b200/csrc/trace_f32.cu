@@ -40,14 +40,14 @@ int fast_grid(FastKernel kernel, int device, int block, size_t smem, int64_t tot
 
 // Workspace layout for a float32 batch (each part 256-aligned):
 //   [0] chunk counter | group queue counters u64[G] | ray prefix int64[J+1] | Job<float>[J] |
-//   FinalizeTargets[J] | FastGroup[G] | FastChunk[NC] | group chunk prefix int64[G+1] | group ray prefix int64[G+1]
+//   FinalizeTargets[J] | FastGroup[G] | group ray prefix int64[G+1]
 // Everything from the ray prefix on is staged on the host and copied in one transfer; the counters are zeroed
 // on the device.
 struct F32Layout {
-    size_t queues, prefix, jobs, targets, groups, chunks, group_chunks, group_rays, total;
+    size_t queues, prefix, jobs, targets, groups, group_rays, total;
 };
 
-F32Layout f32_layout(int32_t jobs, int64_t groups, int64_t chunks) {
+F32Layout f32_layout(int32_t jobs, int64_t groups) {
     F32Layout l{};
     size_t off = 256;
     l.queues = off;       off = align256(off + sizeof(unsigned long long) * static_cast<size_t>(groups));
@@ -55,8 +55,6 @@ F32Layout f32_layout(int32_t jobs, int64_t groups, int64_t chunks) {
     l.jobs = off;         off = align256(off + sizeof(Job<float>) * static_cast<size_t>(jobs));
     l.targets = off;      off = align256(off + sizeof(FinalizeTargets) * static_cast<size_t>(jobs));
     l.groups = off;       off = align256(off + sizeof(FastGroup) * static_cast<size_t>(groups));
-    l.chunks = off;       off = align256(off + sizeof(FastChunk) * static_cast<size_t>(chunks));
-    l.group_chunks = off; off = align256(off + sizeof(int64_t) * (static_cast<size_t>(groups) + 1));
     l.group_rays = off;   off = align256(off + sizeof(int64_t) * (static_cast<size_t>(groups) + 1));
     l.total = off;
     return l;
@@ -71,22 +69,15 @@ std::vector<int32_t> scene_order(const ac_job *jobs, const int32_t *indices, int
     return order;
 }
 
-void count_groups_chunks(const ac_job *jobs, const std::vector<int32_t> &order, int64_t chunk_rays, int64_t *groups,
-                         int64_t *chunks) {
-    *groups = 0;
-    *chunks = 0;
+int64_t count_groups(const ac_job *jobs, const std::vector<int32_t> &order) {
+    int64_t groups = 0;
     size_t k = 0;
     while (k < order.size()) {
         const ac_scene_t scene = jobs[order[k]].scene;
-        int64_t rays = 0;
-        int64_t members = 0;
-        while (k < order.size() && jobs[order[k]].scene == scene && members < kMaxGroupJobs) {
-            rays += jobs[order[k++]].params.num_rays;
-            ++members;
-        }
-        *groups += 1;
-        *chunks += (rays + chunk_rays - 1) / chunk_rays;
+        for (int64_t members = 0; k < order.size() && jobs[order[k]].scene == scene && members < kMaxGroupJobs; ++members) ++k;
+        ++groups;
     }
+    return groups;
 }
 
 }  // namespace
@@ -129,11 +120,8 @@ int launch_trace_f32(const ac_scene_s *scene, const ac_trace_params *p, const ac
     return launch_finalize_single<float>(scene, p, o, scale, stream_ptr);
 }
 
-size_t batch_workspace_bytes_f32(const ac_job *jobs, const int32_t *indices, int32_t count, const ac_batch_config *cfg) {
-    const int64_t chunk_rays = (cfg && cfg->chunk_rays > 0) ? cfg->chunk_rays : kDefaultChunkRays;
-    int64_t groups = 0, chunks = 0;
-    count_groups_chunks(jobs, scene_order(jobs, indices, count), chunk_rays, &groups, &chunks);
-    return f32_layout(count, groups, chunks).total;
+size_t batch_workspace_bytes_f32(const ac_job *jobs, const int32_t *indices, int32_t count, const ac_batch_config *) {
+    return f32_layout(count, count_groups(jobs, scene_order(jobs, indices, count))).total;
 }
 
 int launch_batch_f32(const ac_job *jobs_in, const int32_t *indices, int32_t count, const ac_batch_config *cfg,
@@ -141,9 +129,8 @@ int launch_batch_f32(const ac_job *jobs_in, const int32_t *indices, int32_t coun
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
     const int64_t chunk_rays = (cfg && cfg->chunk_rays > 0) ? cfg->chunk_rays : kDefaultChunkRays;
     const std::vector<int32_t> order = scene_order(jobs_in, indices, count);
-    int64_t num_groups = 0, num_chunks = 0;
-    count_groups_chunks(jobs_in, order, chunk_rays, &num_groups, &num_chunks);
-    const F32Layout l = f32_layout(count, num_groups, num_chunks);
+    const int64_t num_groups = count_groups(jobs_in, order);
+    const F32Layout l = f32_layout(count, num_groups);
     if (workspace_bytes < l.total)
         return fail(AC_ERR_CAPACITY, "batch workspace too small: %zu < %zu", workspace_bytes, l.total);
     std::vector<unsigned char> local;
@@ -156,29 +143,19 @@ int launch_batch_f32(const ac_job *jobs_in, const int32_t *indices, int32_t coun
     Job<float> *jobs = reinterpret_cast<Job<float> *>(host + l.jobs);
     FinalizeTargets *targets = reinterpret_cast<FinalizeTargets *>(host + l.targets);
     FastGroup *groups = reinterpret_cast<FastGroup *>(host + l.groups);
-    FastChunk *chunks = reinterpret_cast<FastChunk *>(host + l.chunks);
-    int64_t *group_chunks = reinterpret_cast<int64_t *>(host + l.group_chunks);
     int64_t *group_rays = reinterpret_cast<int64_t *>(host + l.group_rays);
     int device = -1, need = 0;
-    int64_t total = 0, g = -1, c = 0;
+    int64_t total = 0, g = -1;
     const ac_scene_s *current = nullptr;
-    int64_t group_begin = 0;
-    auto close_group = [&](int64_t group_end) {
-        group_chunks[g] = c;
-        group_rays[g] = group_begin;
-        for (int64_t b = group_begin; b < group_end; b += chunk_rays)
-            chunks[c++] = FastChunk{b, std::min(b + chunk_rays, group_end), static_cast<int32_t>(g), 0};
-    };
     for (int32_t k = 0; k < count; ++k) {
         const ac_job &in = jobs_in[order[k]];
         if (device < 0) device = in.scene->device;
         if (in.scene->device != device) return fail(AC_ERR_INVALID, "batch jobs must share one device");
         if (in.scene->fast.num_bvh_nodes > 0) need = std::max(need, in.scene->bvh_stack_need);
         if (in.scene != current || groups[g].num_jobs >= kMaxGroupJobs) {
-            if (g >= 0) close_group(total);
             ++g;
             current = in.scene;
-            group_begin = total;
+            group_rays[g] = total;
             groups[g] = FastGroup{in.scene->f32, in.scene->fast, k, 0};
         }
         groups[g].num_jobs += 1;
@@ -196,12 +173,10 @@ int launch_batch_f32(const ac_job *jobs_in, const int32_t *indices, int32_t coun
         targets[k] = FinalizeTargets{in.outputs.echogram, in.params.render_ambisonics ? in.outputs.ambisonic : nullptr,
                                      in.outputs.surface_energy};
     }
-    if (g >= 0) close_group(total);
     int entries = 0;
     const int rc = launch_stack_entries(cfg ? cfg->stack_entries : 0, need, &entries);
     if (rc != AC_OK) return rc;
     prefix[count] = total;
-    group_chunks[num_groups] = c;
     group_rays[num_groups] = total;
     AC_CUDA_TRY(cudaSetDevice(device));
     unsigned char *ws = static_cast<unsigned char *>(workspace);
@@ -222,13 +197,10 @@ int launch_batch_f32(const ac_job *jobs_in, const int32_t *indices, int32_t coun
         table.jobs = d_jobs;
         table.ray_begin = reinterpret_cast<const int64_t *>(ws + l.prefix);
         table.groups = reinterpret_cast<const FastGroup *>(ws + l.groups);
-        table.chunks = reinterpret_cast<const FastChunk *>(ws + l.chunks);
-        table.num_chunks = num_chunks;
         table.num_jobs = count;
         table.chunk_rays = static_cast<int32_t>(chunk_rays);
         table.chunk_counter = counter;
         table.group_next = reinterpret_cast<unsigned long long *>(ws + l.queues);
-        table.group_chunk_begin = reinterpret_cast<const int64_t *>(ws + l.group_chunks);
         table.group_ray_begin = reinterpret_cast<const int64_t *>(ws + l.group_rays);
         table.num_groups = static_cast<int32_t>(num_groups);
         Job<float> unused;

@@ -75,13 +75,6 @@ struct FastGroup {
     int32_t num_jobs;
 };
 
-struct FastChunk {
-    int64_t begin;
-    int64_t end;
-    int32_t group;
-    int32_t pad;
-};
-
 // Continuous batching (ac_service_*): a ring of job slots in device memory that
 // the host appends to while a persistent launch runs.  A slot is written once
 // per job before the job is published and not rewritten while a launch that
@@ -116,10 +109,9 @@ struct FastTable {
     const Job<float> *jobs;
     const int64_t *ray_begin;      // [num_jobs + 1]
     const FastGroup *groups;
-    const FastChunk *chunks;       // group by group
-    int64_t num_chunks;
     int32_t num_jobs;
-    int32_t chunk_rays;            // single-job launches: rays per chunk
+    int32_t chunk_rays;            // rays per chunk: chunk k of a group (or of the single job) holds its rays
+                                   // k * chunk_rays onward
     unsigned long long *chunk_counter;   // single-job launches: next chunk
     // Batched launches: one chunk queue per scene group.  A warp starts on the
     // group that holds its share of the rays and stays on it until the group's
@@ -127,7 +119,6 @@ struct FastTable {
     // drains its lanes for a change of scene about once per group it visits,
     // not at every group boundary of one shared queue.
     unsigned long long *group_next;      // [num_groups] chunks taken from each group
-    const int64_t *group_chunk_begin;    // [num_groups + 1] first chunk of each group
     const int64_t *group_ray_begin;      // [num_groups + 1] first ray (over all jobs) of each group
     int32_t num_groups;
     int32_t reserved;
@@ -869,7 +860,7 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
     // slots) during the traversal.  Every lane stores the same values.
     struct WarpWork {
         long long next, end;   // rays next .. end - 1 of the current chunk are not handed out yet
-        long long pending;     // chunk of another scene, taken but not started (-1: none)
+        long long pending;     // chunk of another scene (batched: of group `queue`), taken but not started (-1: none)
         int group;             // the scene group (service launches: the slot) the warp's lanes trace
         int queue;             // batched launches: the group queue this warp takes chunks from
         int exhausted;
@@ -877,7 +868,7 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
     __shared__ WarpWork warp_work[8];
     volatile WarpWork &ww = warp_work[threadIdx.x >> 5];
     ww.next = 0; ww.end = 0; ww.pending = -1; ww.group = -1; ww.queue = 0; ww.exhausted = 0;
-    const int64_t num_chunks = kSingle ? (single.num_rays + table.chunk_rays - 1) / table.chunk_rays : table.num_chunks;
+    const int64_t num_chunks = kSingle ? (single.num_rays + table.chunk_rays - 1) / table.chunk_rays : 0;
     // Service launches: the warp's job-ring state lives in shared memory and is read where it is used, so it
     // holds no registers across the traversal (every lane stores the same values).
     struct ServiceWarp {
@@ -943,6 +934,11 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
         }
         ww.queue = lo;
     }
+
+    auto chunk_range = [&](int g, int64_t k, int64_t &begin, int64_t &stop) {   // rays of chunk k of group g
+        begin = __ldg(table.group_ray_begin + g) + k * table.chunk_rays;
+        stop = min(begin + table.chunk_rays, __ldg(table.group_ray_begin + g + 1));
+    };
 
     FastLane s;
     __shared__ LaneShared lane_shared;
@@ -1016,13 +1012,12 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
                     while (true) {
                         if (lane_id == 0) {
                             c = -1;
-                            const int64_t first = __ldg(table.group_chunk_begin + queue);
-                            const int64_t count = __ldg(table.group_chunk_begin + queue + 1) - first;
+                            const int64_t rays = __ldg(table.group_ray_begin + queue + 1) - __ldg(table.group_ray_begin + queue);
                             const unsigned long long taken =
                                 *reinterpret_cast<volatile unsigned long long *>(table.group_next + queue);
-                            if (static_cast<int64_t>(taken) < count) {
+                            if (static_cast<int64_t>(taken) * table.chunk_rays < rays) {
                                 const int64_t k = static_cast<int64_t>(atomicAdd(table.group_next + queue, 1ull));
-                                if (k < count) c = first + k;
+                                if (k * table.chunk_rays < rays) c = k;
                             }
                         }
                         c = __shfl_sync(full, c, 0);
@@ -1039,8 +1034,8 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
                         ce = min(cb + static_cast<int64_t>(table.chunk_rays), single.num_rays);
                         cg = 0;
                     } else {
-                        const FastChunk ch = table.chunks[c];
-                        cb = ch.begin; ce = ch.end; cg = ch.group;
+                        chunk_range(queue, c, cb, ce);
+                        cg = queue;
                     }
                     if (group >= 0 && cg != group) {
                         if (!__any_sync(full, has)) {
@@ -1104,8 +1099,8 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
                 if (kService) {
                     group = static_cast<int>(pending); cur_slot = group; next = pending_begin; end = pending_end;
                 } else {
-                    const FastChunk ch = table.chunks[pending];
-                    group = ch.group; next = ch.begin; end = ch.end;
+                    group = queue;   // the queue that the chunk came from
+                    chunk_range(queue, pending, next, end);
                 }
                 pending = -1;
                 save();
