@@ -127,6 +127,7 @@ int ensure_launch(ac_service_s *s) {
     slot->first = first;
     slot->window_end = first + s->capacity / 2;
     ac::FastTable t{};
+    t.lanes = 32;
     t.slots = s->slots;
     t.slot_state = s->state;
     t.control = s->control_dev;

@@ -121,7 +121,12 @@ struct FastTable {
     unsigned long long *group_next;      // [num_groups] chunks taken from each group
     const int64_t *group_ray_begin;      // [num_groups + 1] first ray (over all jobs) of each group
     int32_t num_groups;
-    int32_t reserved;
+    int32_t lanes;                 // lanes of a warp that take rays (launches with few rays spread them over more warps)
+    // Single-job launches: the accumulators of the block lie in shared memory behind the traversal stacks
+    // (shared_cells cells of four words, then two counters per surface) and are added to the outputs when it ends;
+    // 0: every deposit goes to the outputs.
+    int32_t shared_cells;
+    int32_t stack_words;           // 32-bit words of the traversal stacks
     // Service launches (continuous batching): the ring, its per-slot state and the control block.
     const ServiceSlot *slots;
     ServiceSlotState *slot_state;
@@ -303,9 +308,6 @@ __device__ __forceinline__ void service_finish(const FastTable &t, int slot, int
 // each (t = v * inv - o * inv); measured 2-4 % faster than (v - o) * inv on the
 // U room and the 8-room apartment, with identical results (node boxes are
 // padded, so the culling stays conservative under either rounding).
-#ifndef AC_WARP_DEPOSIT
-#define AC_WARP_DEPOSIT 0
-#endif
 #ifndef AC_FMA_SLAB
 #define AC_FMA_SLAB 1
 #endif
@@ -787,6 +789,105 @@ __device__ __forceinline__ void winner_normal(const SceneDev<float> &sc, int si,
     if (n[0] * r.d[0] + n[1] * r.d[1] + n[2] * r.d[2] > 0.0f) { n[0] = -n[0]; n[1] = -n[1]; n[2] = -n[2]; }
 }
 
+// A block's own accumulators of a single-job launch, in shared memory: per cell the sum of the quanta's low halves and
+// the sum of their high halves, each as two 32-bit words (the same sums that add_fixed forms in the outputs), then the
+// hit and contribution counts of the surfaces.  Cells: the echogram [6, bins], the three directional ambisonic channels
+// [6, 3, bins], the surfaces' energies.  All rays of a small room deposit into a few hundred addresses, and at L2 those
+// atomics queue up behind one another (shoebox, 100 bins, 50 bounces: 100,000 rays 3.57 ms into the outputs, 0.43 here;
+// 400,000 rays 13.3 and 1.28).
+struct SharedSums {
+    unsigned *words;
+    int cells;
+
+    __device__ __forceinline__ explicit SharedSums(const FastTable &t) : cells(t.shared_cells) {
+        extern __shared__ int stack_words[];
+        words = reinterpret_cast<unsigned *>(stack_words) + t.stack_words;
+    }
+
+    __device__ __forceinline__ void add(int cell, long long q) const {
+        if (q == 0) return;
+        const unsigned lo = static_cast<unsigned>(q), hi = static_cast<unsigned>(q >> 32);
+        unsigned *w = words + cell;
+        if (lo) {
+            const unsigned old = atomicAdd(w, lo);
+            if (old + lo < old) atomicAdd(w + cells, 1u);
+        }
+        unsigned top = q < 0 ? 0xFFFFFFFFu : 0u;   // the high half is signed
+        if (hi) {
+            const unsigned old = atomicAdd(w + 2 * cells, hi);
+            top += old + hi < old ? 1u : 0u;
+        }
+        if (top) atomicAdd(w + 3 * cells, top);
+    }
+
+    __device__ __forceinline__ unsigned *hits() const { return words + 4 * cells; }
+
+    // Adds the block's sums to the job's outputs.
+    __device__ __forceinline__ void flush(const Job<float> &job) const {
+        const int bins = job.num_bins, echo = kBands * bins, surfaces = job.scene.num_surfaces;
+        for (int i = threadIdx.x; i < cells; i += blockDim.x) {
+            const unsigned long long w0 = words[i] | static_cast<unsigned long long>(words[i + cells]) << 32;
+            const unsigned long long w1 =
+                words[i + 2 * cells] | static_cast<unsigned long long>(words[i + 3 * cells]) << 32;
+            unsigned long long *out;
+            if (i < echo) {
+                out = job.echogram_fx + 2 * i;
+            } else if (i < cells - surfaces) {
+                const int a = i - echo, band = a / (3 * bins), rest = a - band * 3 * bins;
+                out = job.ambisonic_fx + 2 * (static_cast<size_t>(band) * 4 * bins + bins + rest);
+            } else {
+                out = job.surface_energy_fx + 2 * (i - (cells - surfaces));
+            }
+            if (w0) atomicAdd(out, w0);
+            if (w1) atomicAdd(out + 1, w1);
+        }
+        for (int i = threadIdx.x; i < surfaces; i += blockDim.x) {
+            const unsigned h = hits()[i], c = hits()[surfaces + i];
+            if (h) atomicAdd(job.hit_counts + i, static_cast<unsigned long long>(h));
+            if (c) atomicAdd(job.contrib_counts + i, static_cast<unsigned long long>(c));
+        }
+    }
+};
+
+// Where a lane's deposits go: the block's shared accumulators, or the job's accumulators in global memory (in a batch
+// the block's copy of them, see Job::shard_mask).
+template <bool kSingle, bool kShards>
+struct Deposit {
+    const Job<float> &job;
+    const FastTable &table;
+    size_t shard;
+
+    __device__ __forceinline__ Deposit(const Job<float> &j, const FastTable &t) : job(j), table(t), shard(0) {
+        if (kShards) shard = static_cast<size_t>(blockIdx.x & job.shard_mask) * job.shard_stride;
+    }
+    __device__ __forceinline__ bool shared() const { return kSingle && table.shared_cells > 0; }
+
+    // Echogram cell band * bins + bin.
+    __device__ __forceinline__ void add(int cell, long long q) const {
+        if (shared()) SharedSums(table).add(cell, q);
+        else add_fixed(job.echogram_fx + shard + 2 * static_cast<size_t>(cell), q);
+    }
+    // Directional ambisonic channel 1 + axis of a band and bin; `cell`: its shared cell.
+    __device__ __forceinline__ void add_direction(int cell, int band, int axis, int bin, long long q) const {
+        if (shared()) SharedSums(table).add(cell, q);
+        else add_fixed(job.ambisonic_fx + shard + 2 * (static_cast<size_t>(band * 4 + 1 + axis) * job.num_bins + bin), q);
+    }
+    __device__ __forceinline__ void add_surface(int surf, long long energy) const {
+        if (shared()) {
+            const SharedSums sums(table);
+            atomicAdd(sums.hits() + job.scene.num_surfaces + surf, 1u);
+            sums.add(sums.cells - job.scene.num_surfaces + surf, energy);
+        } else {
+            atomicAdd(job.contrib_counts + shard + surf, 1ull);
+            add_fixed(job.surface_energy_fx + shard + 2 * static_cast<size_t>(surf), energy);
+        }
+    }
+    __device__ __forceinline__ void add_hits(int surf, unsigned count) const {
+        if (shared()) atomicAdd(SharedSums(table).hits() + surf, count);
+        else atomicAdd(job.hit_counts + shard + surf, static_cast<unsigned long long>(count));
+    }
+};
+
 // The reference's escape-link walk, kept out of line: only rays that miss
 // every surface in BVH mode take it.
 static __device__ __noinline__ int2 fallback_walk(const SceneDev<float> sc, float ox, float oy, float oz, float dx,
@@ -847,7 +948,7 @@ __device__ __forceinline__ int find_job_range(const int64_t *prefix, int lo, int
     return lo;
 }
 
-template <bool kSingle, bool kPhilox, bool kAmb, bool kVisual, bool kService = false>
+template <bool kSingle, bool kPhilox, bool kAmb, bool kVisual, bool kService = false, bool kShards = false>
 __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(const __grid_constant__ Job<float> single,
                                                          const __grid_constant__ FastScene single_fast,
                                                          const __grid_constant__ FastTable table) {
@@ -948,6 +1049,12 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
     volatile long long &lane_ray = lane_shared.ray[threadIdx.x];
     bool has = false;
     s.job = 0;
+    const bool takes = lane_id < table.lanes;
+    if (kSingle && table.shared_cells > 0) {
+        SharedSums sums(table);
+        for (int i = threadIdx.x; i < 4 * table.shared_cells + 2 * single.scene.num_surfaces; i += blockDim.x) sums.words[i] = 0u;
+        __syncthreads();
+    }
 
     while (true) {
         int group = ww.group, queue = ww.queue;
@@ -959,7 +1066,7 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
             ww.exhausted = exhausted ? 1 : 0;
         };
         // ---- refill lanes from the warp's range; take more chunks of the same scene as needed
-        unsigned need = __ballot_sync(full, !has);
+        unsigned need = __ballot_sync(full, !has && takes);
         while (need && pending < 0 && !exhausted) {
             if (next >= end) {
                 long long c = 0;
@@ -1052,7 +1159,7 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
             const int take = static_cast<int>(min(static_cast<int64_t>(__popc(need)), end - next));
             // the `take` lowest needing lanes get rays next .. next+take-1
             const int rank = __popc(need & lanes_below);
-            if (!has && rank < take) {
+            if (!has && takes && rank < take) {
                 const int64_t g = next + rank;
                 int j = 0;
                 int64_t ri = g;
@@ -1092,7 +1199,7 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
                 }
             }
             next += take;
-            need = __ballot_sync(full, !has);
+            need = __ballot_sync(full, !has && takes);
         }
         if (!__any_sync(full, has)) {
             if (pending >= 0) {
@@ -1201,7 +1308,7 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
                              : __match_any_sync(counting, ((static_cast<unsigned>(s.job) & 1023u) << 22) |
                                                               static_cast<unsigned>(surf));
                 if (lane_id == __ffs(same) - 1)
-                    atomicAdd(job.hit_counts + surf, static_cast<unsigned long long>(__popc(same)));
+                    Deposit<kSingle, kShards>(job, table).add_hits(surf, static_cast<unsigned>(__popc(same)));
             }
             const float h[3] = {hx, hy, hz};
             make_ray(query, h, sd);
@@ -1239,63 +1346,23 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
                         const float common = job.ray_scale * source_gain * distance_term * (diffuse + specular);
                         long long esum = 0;
                         float energy_sum = 0.0f;
-#if AC_WARP_DEPOSIT
-                        // lanes depositing into the same (job, bin) add their quanta in the warp first and one of
-                        // them issues the two atomics of each band (quanta are non-negative and below 2^62, so
-                        // their 16-bit pieces sum exactly in 32 bits)
-                        const unsigned dep_mask = __activemask();
-                        const unsigned dep_same =
-                            kService ? __match_any_sync(dep_mask, (static_cast<unsigned long long>(s.job) << 32) |
-                                                                      static_cast<unsigned>(bin))
-                                     : __match_any_sync(dep_mask, ((static_cast<unsigned>(s.job) & 1023u) << 21) |
-                                                                      static_cast<unsigned>(bin));
-                        const bool dep_alone = kAmb || __popc(dep_same) == 1;
-                        const bool dep_leader = lane_id == __ffs(dep_same) - 1;
-#endif
+                        const Deposit<kSingle, kShards> deposit(job, table);
 #pragma unroll
                         for (int b = 0; b < kBands; ++b) {
                             const float e = common * refl[b] * lane_acc[b * kStackStride];
                             if (kVisual) energy_sum += e;
                             const long long qe = quantize(e, job.energy_scale);
-#if AC_WARP_DEPOSIT
-                            if (dep_alone) {
-                                add_fixed(job.echogram_fx + 2 * (static_cast<size_t>(b) * job.num_bins + bin), qe);
-                            } else {
-                                const unsigned long long uq = static_cast<unsigned long long>(qe);
-                                const unsigned l0 = __reduce_add_sync(dep_same, static_cast<unsigned>(uq & 0xFFFFu));
-                                const unsigned l1 =
-                                    __reduce_add_sync(dep_same, static_cast<unsigned>((uq >> 16) & 0xFFFFu));
-                                const unsigned h0 =
-                                    __reduce_add_sync(dep_same, static_cast<unsigned>((uq >> 32) & 0xFFFFu));
-                                const unsigned h1 = __reduce_add_sync(dep_same, static_cast<unsigned>(uq >> 48));
-                                if (dep_leader) {
-                                    unsigned long long *w =
-                                        job.echogram_fx + 2 * (static_cast<size_t>(b) * job.num_bins + bin);
-                                    const unsigned long long lo = static_cast<unsigned long long>(l0) +
-                                                                  (static_cast<unsigned long long>(l1) << 16);
-                                    const unsigned long long hi = static_cast<unsigned long long>(h0) +
-                                                                  (static_cast<unsigned long long>(h1) << 16);
-                                    if (lo) atomicAdd(w, lo);
-                                    if (hi) atomicAdd(w + 1, hi);
-                                }
-                            }
-#else
-                            add_fixed(job.echogram_fx + 2 * (static_cast<size_t>(b) * job.num_bins + bin), qe);
-#endif
-                            if (kAmb) {
+                            deposit.add(b * job.num_bins + bin, qe);
+                            if (kAmb) {   // the W channel is the echogram's own sums: the launch's last kernel copies them
                                 const float *d0 = s.d0;
-                                unsigned long long *a =
-                                    job.ambisonic_fx + 2 * (static_cast<size_t>(b) * 4 * job.num_bins + bin);
-                                const size_t stride = 2 * static_cast<size_t>(job.num_bins);
-                                add_fixed(a, qe);
-                                add_fixed(a + stride, quantize(e * d0[0], job.energy_scale));
-                                add_fixed(a + 2 * stride, quantize(e * d0[1], job.energy_scale));
-                                add_fixed(a + 3 * stride, quantize(e * d0[2], job.energy_scale));
+                                const int a = kBands * job.num_bins + b * 3 * job.num_bins + bin;
+                                deposit.add_direction(a, b, 0, bin, quantize(e * d0[0], job.energy_scale));
+                                deposit.add_direction(a + job.num_bins, b, 1, bin, quantize(e * d0[1], job.energy_scale));
+                                deposit.add_direction(a + 2 * job.num_bins, b, 2, bin, quantize(e * d0[2], job.energy_scale));
                             }
                             esum += qe;
                         }
-                        atomicAdd(job.contrib_counts + surf, 1ull);
-                        add_fixed(job.surface_energy_fx + 2 * static_cast<size_t>(surf), esum);
+                        deposit.add_surface(surf, esum);
                         if (kVisual && s.vslot >= 0)
                             visual_contribution(job, s.vslot, s.bounce, energy_sum,
                                                 static_cast<float>(s.path + static_cast<double>(t) +
@@ -1386,6 +1453,10 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
         const int cs = count_slot;
         const unsigned long long cn = count_n;
         if (cn && service_count(table, cs, cn, lane_id)) service_finish(table, cs, lane_id);
+    }
+    if (kSingle && table.shared_cells > 0) {
+        __syncthreads();   // every warp of the block has made its last deposit
+        SharedSums(table).flush(single);
     }
 }
 

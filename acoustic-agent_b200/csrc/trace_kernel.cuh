@@ -151,6 +151,10 @@ struct Job {
     int32_t *visual_orders;            // [L]
     T *visual_distances;               // [L]
     T *visual_gains;                   // [L]
+    // float32 batches: the job's accumulators above lie in a workspace region of shard_mask + 1 copies, shard_stride
+    // words apart, which the blocks share out; 0: they are the caller's outputs themselves
+    int32_t shard_mask;
+    int64_t shard_stride;
 };
 
 // Visual slot of a ray, -1 for none (steam_rt.py:4726-4731).
