@@ -34,10 +34,11 @@ struct Offsets {
         box_bounds, boxes, edges, bvh_nodes, bvh_prims, total;  // elements
 };
 
-// Scenes with more walls + boxes than this trace in BVH mode unless the caller chooses;
-// with at most kAutoHybridWalls walls (one room) in hybrid mode.  Measured on B200:
-// U room (8 walls, 20 boxes) hybrid 11.4 ms < BVH 11.8 < scan 12.3; 8-room apartment
-// (52 walls, 374 boxes) BVH 5.1 ms < hybrid 6.3 < scan 9.6.
+// Unless the caller chooses, a single room (at most kAutoHybridWalls walls) with any box traces in hybrid mode, its walls
+// in lockstep and its boxes in a BVH; other scenes of more than kAutoBvhSurfaces walls and boxes in BVH mode.  Measured on
+// B200: a 4-wall room, 10,000 / 400,000 rays: with 1 box scan 0.466 / 2.24 ms, hybrid 0.456 / 2.19, with 12 boxes scan
+// 0.668 / 2.60, hybrid 0.554 / 2.27, BVH 0.548 / 2.46; U room (8 walls, 20 boxes) hybrid 11.4 ms < BVH 11.8 < scan 12.3;
+// 8-room apartment (52 walls, 374 boxes) BVH 5.1 ms < hybrid 6.3 < scan 9.6 (the last two by earlier kernels).
 constexpr int64_t kAutoBvhSurfaces = 16;
 constexpr int64_t kAutoHybridWalls = 16;
 // Float32 BVH node boxes are padded by this much (metres) beyond the surface bounds, or by 4e-7 of the largest
@@ -461,8 +462,7 @@ extern "C" int ac_scene_create(const ac_scene_desc *d, ac_scene_t *out) {
             }
             // AUTO: a single room's few walls are cheapest in lockstep, its furniture in a BVH
             lists.hybrid = d->traversal == AC_TRAVERSAL_HYBRID ||
-                           (d->traversal == AC_TRAVERSAL_AUTO && walls + boxes > kAutoBvhSurfaces &&
-                            walls <= kAutoHybridWalls && boxes > 0);
+                           (d->traversal == AC_TRAVERSAL_AUTO && walls <= kAutoHybridWalls && boxes > 0);
             std::vector<int64_t> members;
             for (int64_t i = 0; i < S; ++i)
                 if (d->kinds[i] == AC_KIND_BOX || (d->kinds[i] == AC_KIND_WALL && !lists.hybrid)) members.push_back(i);

@@ -118,25 +118,30 @@ __global__ void finalize_f32_kernel(const Job<float> *jobs, const FinalizeTarget
 
 using FastKernel = void (*)(const Job<float>, const FastScene, const FastTable);
 
-template <bool kSingle, bool kVisual>
-FastKernel pick_variant(bool philox, bool amb) {
+template <bool kSingle, bool kVisual, bool kShards, bool kLean>
+FastKernel pick_stream(bool philox, bool amb) {
     if (philox)
-        return amb ? trace_fast_kernel<kSingle, true, true, kVisual> : trace_fast_kernel<kSingle, true, false, kVisual>;
-    return amb ? trace_fast_kernel<kSingle, false, true, kVisual> : trace_fast_kernel<kSingle, false, false, kVisual>;
+        return amb ? trace_fast_kernel<kSingle, true, true, kVisual, false, kShards, kLean>
+                   : trace_fast_kernel<kSingle, true, false, kVisual, false, kShards, kLean>;
+    return amb ? trace_fast_kernel<kSingle, false, true, kVisual, false, kShards, kLean>
+               : trace_fast_kernel<kSingle, false, false, kVisual, false, kShards, kLean>;
+}
+
+template <bool kSingle, bool kLean>
+FastKernel pick_variant(bool philox, bool amb, bool visual, bool shards) {
+    if (visual) return pick_stream<kSingle, true, false, kLean>(philox, amb);
+    return !kSingle && shards ? pick_stream<kSingle, false, !kSingle, kLean>(philox, amb)
+                              : pick_stream<kSingle, false, false, kLean>(philox, amb);
 }
 
 template <bool kSingle>
-FastKernel pick_kernel(bool philox, bool amb, bool visual) {
-    return visual ? pick_variant<kSingle, true>(philox, amb) : pick_variant<kSingle, false>(philox, amb);
+FastKernel pick_kernel(bool philox, bool amb, bool visual, bool shards, bool lean) {
+    return lean ? pick_variant<kSingle, true>(philox, amb, visual, shards)
+                : pick_variant<kSingle, false>(philox, amb, visual, shards);
 }
 
-FastKernel pick_sharded(bool philox, bool amb) {
-    if (philox)
-        return amb ? trace_fast_kernel<false, true, true, false, false, true>
-                   : trace_fast_kernel<false, true, false, false, false, true>;
-    return amb ? trace_fast_kernel<false, false, true, false, false, true>
-               : trace_fast_kernel<false, false, false, false, false, true>;
-}
+// Whether the lean kernels can trace a scene: no boxes in the lockstep scan, no four-wide BVH.
+bool scene_is_lean(const FastScene &f) { return f.num_box_clusters == 0 && (f.num_bvh_nodes == 0 || f.bvh_width == 2); }
 
 int fast_grid(FastKernel kernel, int device, int block, size_t smem, int64_t total_rays, int requested) {
     int per_sm = 0;
@@ -269,7 +274,7 @@ int launch_trace_f32(const ac_scene_s *scene, const ac_trace_params *p, const ac
     table.chunk_counter = reinterpret_cast<unsigned long long *>(o->counters) + 4;
     table.stack_words = static_cast<int32_t>(stack_smem_bytes(entries) / sizeof(int));
     const FastKernel kernel = pick_kernel<true>(p->rng_mode == AC_RNG_PHILOX, p->render_ambisonics != 0,
-                                                p->visual_limit > 0);
+                                                p->visual_limit > 0, false, scene_is_lean(scene->fast));
     size_t smem = stack_smem_bytes(entries);
     {
         const int64_t cells = static_cast<int64_t>(kBands) * p->num_bins * (job.ambisonic_fx ? 4 : 1) + scene->num_surfaces;
@@ -323,6 +328,7 @@ int launch_batch_f32(const ac_job *jobs_in, const int32_t *indices, int32_t coun
     int64_t *group_rays = reinterpret_cast<int64_t *>(host + l.group_rays);
     unsigned long long *shards = reinterpret_cast<unsigned long long *>(static_cast<unsigned char *>(workspace) + l.shards);
     int device = -1, need = 0;
+    bool lean = true;
     int64_t total = 0, g = -1;
     const ac_scene_s *current = nullptr;
     for (int32_t k = 0; k < count; ++k) {
@@ -330,6 +336,7 @@ int launch_batch_f32(const ac_job *jobs_in, const int32_t *indices, int32_t coun
         if (device < 0) device = in.scene->device;
         if (in.scene->device != device) return fail(AC_ERR_INVALID, "batch jobs must share one device");
         if (in.scene->fast.num_bvh_nodes > 0) need = std::max(need, in.scene->bvh_stack_need);
+        lean = lean && scene_is_lean(in.scene->fast);
         if (in.scene != current || groups[g].num_jobs >= kMaxGroupJobs) {
             ++g;
             current = in.scene;
@@ -401,9 +408,8 @@ int launch_batch_f32(const ac_job *jobs_in, const int32_t *indices, int32_t coun
         std::memset(&unused, 0, sizeof(unused));
         FastScene none{};
         // ac_trace_batch partitions jobs so that one launch has one kernel variant.
-        const bool philox = jobs[0].rng_mode == AC_RNG_PHILOX, amb = jobs[0].render_ambisonics != 0;
-        const FastKernel kernel = shard_words ? pick_sharded(philox, amb)
-                                              : pick_kernel<false>(philox, amb, jobs[0].visual_limit > 0);
+        const FastKernel kernel = pick_kernel<false>(jobs[0].rng_mode == AC_RNG_PHILOX, jobs[0].render_ambisonics != 0,
+                                                     jobs[0].visual_limit > 0, shard_words > 0, lean);
         const size_t smem = stack_smem_bytes(entries);
         const int grid = fast_grid(kernel, device, block, smem, spread_rays(total, table.lanes), cfg ? cfg->grid_blocks : 0);
         kernel<<<grid, block, smem, stream>>>(unused, none, table);
