@@ -153,21 +153,6 @@ int fast_grid(FastKernel kernel, int device, int block, size_t smem, int64_t tot
     return grid;
 }
 
-// Lanes of a warp that take rays.  A launch too small to fill the GPU is bound by the time of one warp's bounces, which
-// falls with the lanes it carries (its queries end with the slowest lane's), so its rays are spread over up to two
-// warps per scheduler (furnished U room, 100 bounces: 2,000 rays 0.98 -> 0.77 ms, 10,000 rays 1.06 -> 0.88; with three
-// warps 0.92, and 30,000 rays get slower).  Fewer lanes than `least` gain nothing: 4 where the rays of a warp descend a
-// BVH on their own, 16 in the lockstep scan (shoebox, 10,000 rays 0.36 -> 0.33 ms; 0.35 with 8).
-int warp_lanes(int device, int64_t rays, int least) {
-    const int64_t warps = static_cast<int64_t>(device_sm_count(device)) * 8;
-    return static_cast<int>(std::min<int64_t>(32, std::max<int64_t>(least, (rays + warps - 1) / warps)));
-}
-
-// Rays a launch of full warps would need as many warps for.
-int64_t spread_rays(int64_t rays, int lanes) { return (rays + lanes - 1) / lanes * 32; }
-
-constexpr int kSharedSumBytes = 40 * 1024;   // a block's own accumulators at most: three blocks per SM keep an L1 for the scene
-
 // Words of one copy of a batch job's accumulators.
 size_t accumulator_words(const ac_job &job) {
     const size_t nb = 2 * static_cast<size_t>(kBands) * job.params.num_bins;

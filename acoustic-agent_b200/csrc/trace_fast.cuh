@@ -494,30 +494,31 @@ __device__ __forceinline__ void scene_scan(const FastScene &fs, const FRay &r, b
             if (point_in_polygon_fast(px, py, fs.edges, fs.num_edges) && cand) take(t, si, best_t, best);
         }
     }
-    if (kLean) return;
-    // Boxes: per-lane candidate masks from world AABBs, then per-lane candidates in lockstep.
+    if constexpr (!kLean) {
+        // Boxes: per-lane candidate masks from world AABBs, then per-lane candidates in lockstep.
 #pragma unroll 1
-    for (int c = 0; c < fs.num_box_clusters; ++c) {
-        const bool searching = active && !(any_hit && best >= 0);
-        if (!__any_sync(full, searching)) return;
-        const float *cp = fs.box_clusters + kClusterStride * c;
-        const Quad<float> lo = ldq(cp), hi = ldq(cp + 4);
-        const bool pass = searching && cluster_overlaps(r, lo, hi, best_t);
-        if (!__any_sync(full, pass)) continue;
-        const int first = __float_as_int(lo.w), count = __float_as_int(hi.w);
-        unsigned mask = 0u;
+        for (int c = 0; c < fs.num_box_clusters; ++c) {
+            const bool searching = active && !(any_hit && best >= 0);
+            if (!__any_sync(full, searching)) return;
+            const float *cp = fs.box_clusters + kClusterStride * c;
+            const Quad<float> lo = ldq(cp), hi = ldq(cp + 4);
+            const bool pass = searching && cluster_overlaps(r, lo, hi, best_t);
+            if (!__any_sync(full, pass)) continue;
+            const int first = __float_as_int(lo.w), count = __float_as_int(hi.w);
+            unsigned mask = 0u;
 #pragma unroll 1
-        for (int k = 0; k < count; ++k) {
-            const float *bb = fs.box_bounds + static_cast<size_t>(first + k) * 8;
-            if (pass && cluster_overlaps(r, ldq(bb), ldq(bb + 4), best_t)) mask |= 1u << k;
-        }
-        while (__any_sync(full, mask != 0u)) {
-            if (mask) {
-                const int k = __ffs(mask) - 1;
-                mask &= mask - 1u;
-                const float *rec = fs.boxes + static_cast<size_t>(first + k) * kPrimStride;
-                take(box_t(ldq(rec), ldq(rec + 4), ldq(rec + 8), r), __float_as_int(__ldg(rec + 11)) >> 2, best_t, best);
-                if (any_hit && best >= 0) mask = 0u;
+            for (int k = 0; k < count; ++k) {
+                const float *bb = fs.box_bounds + static_cast<size_t>(first + k) * 8;
+                if (pass && cluster_overlaps(r, ldq(bb), ldq(bb + 4), best_t)) mask |= 1u << k;
+            }
+            while (__any_sync(full, mask != 0u)) {
+                if (mask) {
+                    const int k = __ffs(mask) - 1;
+                    mask &= mask - 1u;
+                    const float *rec = fs.boxes + static_cast<size_t>(first + k) * kPrimStride;
+                    take(box_t(ldq(rec), ldq(rec + 4), ldq(rec + 8), r), __float_as_int(__ldg(rec + 11)) >> 2, best_t, best);
+                    if (any_hit && best >= 0) mask = 0u;
+                }
             }
         }
     }

@@ -321,6 +321,150 @@ __device__ __forceinline__ bool ray_aabb(const T *o, const T *d, const Quad<T> &
 template <typename T>
 __device__ __forceinline__ int rec_tag(const T *rec) { return tag_bits(__ldg(rec + 11)); }
 
+// ---------------------------------------------------------------------------
+// The float64 queries (walk64).  They give the reference's results bit for bit with less work per test:
+//
+//   * a float64 division costs as much as twenty other instructions, and most tests only show that a surface or a node
+//     is not hit.  Quotients by an approximate reciprocal (relative error below 1e-6), or for nodes by the ray's rounded
+//     reciprocals (two rounding steps), settle every test that they clear by a margin far above that error; only the
+//     others do the reference's divisions, whose results are the ones that count;
+//   * in the BVH walk a lane goes on to its next leaf before the warp tests leaves, in the reference's order, so that the
+//     lanes of a warp do the same kind of work;
+//   * the exact tests stand out of line and closest and shadow queries share one walk: inlined twice, the kernel waited
+//     4.7 of 9.2 cycles per instruction for instructions (now 2.2).  A linear scene keeps the inlined loops: with few
+//     surfaces they are short, and out of line a shoebox took 10 % longer at 5,000 rays.
+//
+// What bounds it now is divergence: 3 of 32 lanes are active per instruction.  Measured with the rays of a small launch
+// spread over more warps (warp_lanes): furnished U room in BVH mode, 100 bounces, 500 / 5,000 / 20,000 / 100,000 rays
+// 6.36 / 6.25 / 7.01 / 17.1 -> 2.83 / 3.51 / 5.69 / 11.5 ms; apartment, 2,000 / 20,000 rays 11.6 / 12.7 -> 5.06 / 8.2;
+// shoebox, linear, 50 bounces, 500 / 5,000 / 20,000 rays 0.69 / 0.71 / 1.01 -> 0.56 / 0.71 / 1.02.
+
+__device__ __forceinline__ double approx_inverse(double x) {   // |x| between 1e-30 and 1e30
+    return static_cast<double>(__frcp_rn(static_cast<float>(x)));
+}
+
+// False only if the surface is certainly missed, or hit certainly beyond `limit`.
+__device__ __forceinline__ bool maybe_hit(const double *rec, int kind, const double *o, const double *d, double inv_z,
+                                          double limit) {
+    const Quad<double> A = ldq(rec), B = ldq(rec + 4);
+    if (kind == 0) {
+        const double det = A.z * d[1] - A.w * d[0];
+        if (fabs(det) <= 1e-12) return false;   // the reference's own test
+        const double relx = o[0] - A.x, rely = o[1] - A.y, inv = approx_inverse(det);
+        const double t = (relx * A.w - rely * A.z) * inv, u = (relx * d[1] - rely * d[0]) * inv, z = o[2] + t * d[2];
+        const double clear = 1e-3 + 1e-5 * fabs(t);
+        return t >= -clear && t <= limit + clear && u >= -1e-3 && u <= 1.001 && z >= B.x - clear && z <= B.y + clear;
+    }
+    if (kind == 1) {
+        if (fabs(d[2]) <= 1e-12) return false;   // the reference's own test
+        const double t = (A.x - o[2]) * inv_z, clear = 1e-3 + 1e-5 * fabs(t);
+        return t >= -clear && t <= limit + clear;
+    }
+    const Quad<double> C = ldq(rec + 8);
+    const double relx = o[0] - A.x, rely = o[1] - A.y;
+    double enter = -1e30, leave = 1e30;
+    auto slab = [&](double oo, double dd, double inv, double lo, double hi) {
+        if (fabs(dd) <= 1e-9) return;   // nearly parallel: left to the exact test
+        const double a = (lo - oo) * inv, b = (hi - oo) * inv;
+        enter = fmax(enter, fmin(a, b));
+        leave = fmin(leave, fmax(a, b));
+    };
+    const double dx = d[0] * A.z + d[1] * A.w, dy = d[0] * B.x + d[1] * B.y;
+    slab(relx * A.z + rely * A.w, dx, approx_inverse(dx), -B.z, B.z);
+    slab(relx * B.x + rely * B.y, dy, approx_inverse(dy), -B.w, B.w);
+    slab(o[2], d[2], inv_z, C.x, C.y);
+    const double clear = 1e-3 + 1e-5 * (fabs(enter) + fabs(leave));
+    return enter <= leave + clear && leave >= -clear && enter <= limit + clear;
+}
+
+// The reference's test of one surface, out of line; `n`: its normal at the hit.
+static __device__ __noinline__ double exact_hit(const double *rec, int kind, const double *o, const double *d,
+                                                const double *corners, int num_corners, double *n) {
+    return surface_hit<double>(rec, kind, o, d, corners, num_corners, n);
+}
+
+static __device__ __noinline__ bool exact_node(double ox, double oy, double oz, double dx, double dy, double dz,
+                                               const double *node, double max_distance) {
+    const double o[3] = {ox, oy, oz}, d[3] = {dx, dy, dz};
+    return ray_aabb<double>(o, d, ldq(node), ldq(node + 4), max_distance);
+}
+
+struct Walk64 {
+    double t;
+    int surface;
+};
+
+// Closest query (`any` false, limit 1e30): the nearest surface under the reference's tie rules.  Any query: some surface
+// closer than `limit` (its index, else -1).
+static __device__ __noinline__ Walk64 walk64(const SceneDev<double> &sc, bool any, double ox, double oy, double oz,
+                                             double dx, double dy, double dz, double limit) {
+    const double o[3] = {ox, oy, oz}, d[3] = {dx, dy, dz};
+    const double inv_z = approx_inverse(fabs(dz) < 1e-30 ? 1e-30 : dz);
+    double best_t = limit, n[3];
+    int best = -1;
+    const bool flat = fabs(dx) <= Consts<double>::axis_eps || fabs(dy) <= Consts<double>::axis_eps ||
+                      fabs(dz) <= Consts<double>::axis_eps;
+    const double ix = 1.0 / dx, iy = 1.0 / dy, iz = 1.0 / dz;
+    int node = 0;
+    while (node < sc.num_nodes) {
+        int start = 0, count = 0;
+        while (node < sc.num_nodes) {   // to the next leaf that the ray meets
+            const double *np = sc.nodes + static_cast<size_t>(node) * kNodeStride;
+            const Quad<double> lo = ldq(np), hi = ldq(np + 4);
+            bool meets = false, sure = false;
+            if (!flat) {
+                const double x0 = (lo.x - ox) * ix, x1 = (hi.x - ox) * ix, y0 = (lo.y - oy) * iy, y1 = (hi.y - oy) * iy;
+                const double z0 = (lo.z - oz) * iz, z1 = (hi.z - oz) * iz;
+                const double enter = fmax(fmax(fmin(x0, x1), fmin(y0, y1)), fmax(fmin(z0, z1), 0.0));
+                const double leave = fmin(fmin(fmax(x0, x1), fmax(y0, y1)),
+                                          fmin(fmax(z0, z1), best_t + Consts<double>::bvh_eps));
+                const double clear = 1e-14 * (fabs(enter) + fabs(leave));
+                meets = enter < leave - clear && leave > 1.001e-6;
+                sure = meets || enter > leave + clear || leave < 0.999e-6;
+            }
+            if (!sure) meets = exact_node(ox, oy, oz, dx, dy, dz, np, best_t);
+            if (!meets) {
+                node = tag_bits(lo.w);
+                continue;
+            }
+            ++node;
+            const int bits = tag_bits(hi.w);
+            count = static_cast<int>(static_cast<unsigned>(bits) >> 24);
+            start = bits & 0xFFFFFF;
+            if (count > 0) break;
+        }
+        for (int k = 0; k < count; ++k) {
+            const double *rec = sc.prims_leaf + static_cast<size_t>(start + k) * kPrimStride;
+            const int tag = rec_tag(rec), si = tag >> 2;
+            const double t = maybe_hit(rec, tag & 3, o, d, inv_z, best_t)
+                                 ? exact_hit(rec, tag & 3, o, d, sc.corners, sc.num_corners, n)
+                                 : 1e30;
+            if (any) {
+                if (t < limit) return Walk64{t, si};
+            } else if (t < best_t || (t == best_t && (best < 0 || si < best))) {
+                best_t = t;
+                best = si;
+            }
+        }
+    }
+    return Walk64{best_t, best};
+}
+
+// The hit's normal, oriented against the ray.
+__device__ __forceinline__ void normal64(const SceneDev<double> &sc, int surface, double t, const double *o, const double *d,
+                                         double *n) {
+    if (t == 1e30) {   // the BVH walk's rule for a ray that misses every surface it visits
+        n[0] = __ldg(sc.normals + 3 * surface);
+        n[1] = __ldg(sc.normals + 3 * surface + 1);
+        n[2] = __ldg(sc.normals + 3 * surface + 2);
+    } else {
+        const double *rec = sc.prims_linear + static_cast<size_t>(surface) * kPrimStride;
+        exact_hit(rec, rec_tag(rec) & 3, o, d, sc.corners, sc.num_corners, n);
+    }
+    const double dot = n[0] * d[0] + n[1] * d[1] + n[2] * d[2];
+    if (dot > 0.0) { n[0] = -n[0]; n[1] = -n[1]; n[2] = -n[2]; }
+}
+
 // Closest hit: steam_rt.py:4429-4478 (linear) and :4481-4506 (escape-link walk).
 // The BVH walk keeps the reference's tie rule, including its side effect that a
 // ray missing every visited surface returns the lowest visited index with t=1e30.
@@ -362,8 +506,12 @@ __device__ __forceinline__ int closest_hit(const SceneDev<T> &sc, bool use_bvh, 
             bn[2] = __ldg(sc.normals + 3 * best + 2);
         }
     } else {
+        const double inv_z = approx_inverse(static_cast<double>(fabs(d[2]) < T(1e-30) ? T(1e-30) : d[2]));
         for (int si = 0; si < sc.num_surfaces; ++si) {
             const T *rec = sc.prims_linear + static_cast<size_t>(si) * kPrimStride;
+            if constexpr (sizeof(T) == 8) {
+                if (!maybe_hit(rec, rec_tag(rec) & 3, o, d, inv_z, best_t)) continue;
+            }
             const T t = surface_hit(rec, rec_tag(rec) & 3, o, d, sc.corners, sc.num_corners, n);
             if (t < best_t) { best_t = t; best = si; bn[0] = n[0]; bn[1] = n[1]; bn[2] = n[2]; }
         }
@@ -405,8 +553,12 @@ __device__ __forceinline__ bool any_hit(const SceneDev<T> &sc, bool use_bvh, con
         }
         return false;
     }
+    const double inv_z = approx_inverse(static_cast<double>(fabs(d[2]) < T(1e-30) ? T(1e-30) : d[2]));
     for (int si = 0; si < sc.num_surfaces; ++si) {
         const T *rec = sc.prims_linear + static_cast<size_t>(si) * kPrimStride;
+        if constexpr (sizeof(T) == 8) {
+            if (!maybe_hit(rec, rec_tag(rec) & 3, o, d, inv_z, max_t)) continue;
+        }
         const T t = surface_hit(rec, rec_tag(rec) & 3, o, d, sc.corners, sc.num_corners, n);
         if (t < max_t) return true;
     }
@@ -510,7 +662,7 @@ struct BatchTable {
     const void *jobs;          // Job<T>[num_jobs]
     const int64_t *ray_begin;  // [num_jobs + 1] prefix of num_rays
     int32_t num_jobs;
-    int32_t pad;
+    int32_t lanes;             // lanes of a warp that take rays
     int64_t total_rays;
     unsigned long long *work_counter;
 };
@@ -566,13 +718,13 @@ __global__ void __launch_bounds__(256) trace_kernel(const __grid_constant__ Job<
 
     while (true) {
         // Refill: every lane without a ray takes the next global index.
-        const unsigned need = __ballot_sync(full, !has && !drained);
+        const unsigned need = __ballot_sync(full, !has && !drained && lane_id < table.lanes);
         if (need) {
             const int leader = __ffs(need) - 1;
             unsigned long long base = 0;
             if (lane_id == leader) base = atomicAdd(work_counter, static_cast<unsigned long long>(__popc(need)));
             base = __shfl_sync(full, base, leader);
-            if (!has && !drained) {
+            if (!has && !drained && lane_id < table.lanes) {
                 const int64_t g = static_cast<int64_t>(base) + __popc(need & lanes_below);
                 if (g < total) {
                     int j = 0;
@@ -606,7 +758,7 @@ __global__ void __launch_bounds__(256) trace_kernel(const __grid_constant__ Job<
             }
         }
         if (!__any_sync(full, has)) {
-            if (__all_sync(full, drained || has)) break;
+            if (__all_sync(full, drained || lane_id >= table.lanes)) break;
             continue;
         }
 
@@ -617,8 +769,15 @@ __global__ void __launch_bounds__(256) trace_kernel(const __grid_constant__ Job<
             const Job<T> &job = kSingle ? single : jobs[s.job];
             const SceneDev<T> &sc = job.scene;
             const bool bvh = job.use_bvh != 0;
-            T t, n[3];
-            const int surf = closest_hit(sc, bvh, s.o, s.d, t, n);
+            T t, n[3] = {T(0), T(0), T(0)};
+            int surf;
+            if (bvh) {
+                const Walk64 hit = walk64(sc, false, s.o[0], s.o[1], s.o[2], s.d[0], s.d[1], s.d[2], 1e30);
+                surf = hit.surface;
+                t = hit.t;
+            } else {
+                surf = closest_hit(sc, false, s.o, s.d, t, n);
+            }
             s.queries += 1;
             bool dead = surf < 0 || t <= job.listener_radius || s.path > job.max_path_length;
             if (!dead && s.bounce > 0) {
@@ -631,6 +790,7 @@ __global__ void __launch_bounds__(256) trace_kernel(const __grid_constant__ Job<
                 finished = true;
             } else {
                 count_surface = surf;
+                if (bvh) normal64(sc, surf, t, s.o, s.d, n);
                 if (job.ray_surfaces)
                     job.ray_surfaces[s.ray * job.num_bounces + s.bounce] = surf;
                 const T hx = s.o[0] + t * s.d[0] + T(1e-2) * n[0];
@@ -649,7 +809,11 @@ __global__ void __launch_bounds__(256) trace_kernel(const __grid_constant__ Job<
                     if (facing > T(0)) {
                         const T h[3] = {hx, hy, hz};
                         s.shadows += 1;
-                        const bool occluded = any_hit(sc, bvh, h, sd, dist - T(1e-6));
+                        bool occluded;
+                        if (bvh)
+                            occluded = walk64(sc, true, h[0], h[1], h[2], sd[0], sd[1], sd[2], dist - 1e-6).surface >= 0;
+                        else
+                            occluded = any_hit(sc, false, h, sd, dist - T(1e-6));
                         if (!occluded) {
                             const T diffuse = T(1.0 / kPi) * scat * facing;
                             T half[3];

@@ -55,8 +55,9 @@ enum { AC_RNG_REFERENCE = 0, AC_RNG_PHILOX = 1 };
  * room with tens of surfaces); BVH lets every lane descend its own path of a
  * surface-area-heuristic BVH over walls and boxes with a short stack (best
  * for multi-room scenes with hundreds of surfaces); HYBRID scans the walls in
- * lockstep and descends a BVH over the boxes only; AUTO picks by size (scan
- * up to 16 walls and boxes, hybrid with up to 16 walls, BVH beyond). */
+ * lockstep and descends a BVH over the boxes only; AUTO picks by size (hybrid
+ * with boxes and up to 16 walls, otherwise scan up to 16 walls and boxes, BVH
+ * beyond). */
 enum { AC_TRAVERSAL_AUTO = 0, AC_TRAVERSAL_SCAN = 1, AC_TRAVERSAL_BVH = 2, AC_TRAVERSAL_HYBRID = 3 };
 
 typedef struct ac_scene_s *ac_scene_t;
