@@ -48,6 +48,22 @@ def directivity_gain(direction: Sequence[float], model: Mapping[str, Any]) -> fl
     return float(abs((1.0 - w) + w * c) ** p)
 
 
+def _distances_and_gains(points: np.ndarray, model: Mapping[str, Any]) -> tuple[list[float], list[float]]:
+    """Distance and directivity_gain of [N, 2, 3] source/listener points: the same operations, the model read once
+    (per pair, numpy's overhead on three elements cost 1,024 pairs 14 of 19 ms)."""
+    towards = points[:, 1] - points[:, 0]
+    distances = [math.sqrt(v.dot(v)) for v in towards]
+    forward = source_forward(model)
+    w = float(model.get("dipole_weight", 0.0))
+    p = float(model.get("dipole_power", 1.0))
+    unit = towards / np.maximum(np.asarray(distances), 1e-12).reshape(-1, 1)
+    gains = []
+    for n, v in zip(distances, unit):
+        c = min(max(float(forward.dot(v)), -1.0), 1.0)
+        gains.append(1.0 if n <= 1e-12 else float(abs((1.0 - w) + w * c) ** p))
+    return distances, gains
+
+
 def surface_groups(names: Sequence[str]) -> np.ndarray:
     """Surfaces that share a name share a group: the transmission walk counts each name once."""
     ids: dict[str, int] = {}
@@ -161,52 +177,48 @@ def direct_results(device_scene: runtime.DeviceScene, tables: DirectTables,
                    source_model: str | Mapping[str, Any] | None = None) -> list[dict[str, Any]]:
     """The simulate_direct result dicts for `pairs` of a resident scene and its tables."""
     emitter = source_directivity(source_model)
-    out: list[dict[str, Any]] = []
-    queries = (_lib.ACDirectQuery * max(1, len(pairs)))()
-    traced: list[int] = []
-    geometry = []
-    for source, listener in pairs:
-        src = np.asarray(source, dtype=float)
-        lst = np.asarray(listener, dtype=float)
-        delta = src - lst
-        distance = float(np.linalg.norm(delta))
-        geometry.append((src, lst, distance))
-        if config.direct_occlusion and distance > 1e-6:
-            queries[len(traced)] = make_query(src, lst, config)
-            traced.append(len(geometry) - 1)
-    records = None
-    names = tables.names
+    points = [(np.asarray(source, dtype=float), np.asarray(listener, dtype=float)) for source, listener in pairs]
+    if all(p.shape == (3,) for pair in points for p in pair):
+        coordinates = np.asarray(points, dtype=float).reshape(-1, 2, 3)
+        distances, gains = _distances_and_gains(coordinates, emitter)
+    else:   # what else the formulas take, one pair at a time
+        distances = [float(np.linalg.norm(src - lst)) for src, lst in points]
+        gains = [directivity_gain(lst - src, emitter) for src, lst in points]
+        coordinates = None
+    N = len(points)
+    occlusion, transmission, surface = [1.0] * N, np.ones((N, 6)), [None] * N
+    traced = [g for g in range(N) if config.direct_occlusion and distances[g] > 1e-6]
     if traced:
+        first = make_query(*points[traced[0]], config)
+        queries = (_lib.ACDirectQuery * len(traced))(*[first] * len(traced))
+        table = np.frombuffer(queries, dtype=np.dtype(_lib.ACDirectQuery))
+        asked = (coordinates[traced] if coordinates is not None
+                 else np.stack([np.stack([p.reshape(3) for p in points[g]]) for g in traced]))
+        table["source"], table["listener"] = asked[:, 0], asked[:, 1]
         records = run_queries(device_scene, tables, queries, len(traced),
                               samples=max(1, int(config.direct_occlusion_samples)))
-    slot = {g: k for k, g in enumerate(traced)}
-    for g, (src, lst, distance) in enumerate(geometry):
-        gain = directivity_gain(lst - src, emitter)
-        attenuation = 1.0 / max(distance, config.min_distance_m)
-        air = np.asarray([math.exp(-bands.AIR_ABSORPTION_NP_PER_M[b] * distance) for b in range(6)], dtype=float)
-        occlusion = 1.0
-        transmission = np.ones(6, dtype=float)
-        surface = None
-        if g in slot:
-            rec = records[slot[g]]
-            occlusion = float(rec["occlusion"])
-            surface = names[int(rec["occlusion_surface"])] if int(rec["occlusion_surface"]) >= 0 else None
-            if occlusion < 1.0:
-                transmission = np.asarray(rec["transmission"], dtype=float)
-        band_gains = {band: float(gain * attenuation * air[i] * (occlusion + (1.0 - occlusion) * transmission[i]))
-                      for i, band in enumerate(bands.FREQUENCY_BANDS)}
-        out.append({
-            "distance_m": distance,
-            "delay_s": distance / config.c,
-            "distance_attenuation": attenuation,
-            "air_absorption": air,
-            "occlusion": occlusion,
-            "transmission": transmission,
-            "occlusion_surface": surface,
-            "source_directivity_gain": gain,
-            "band_gains": band_gains,
-        })
-    return out
+        names = tables.names
+        blocked = records["occlusion"] < 1.0
+        transmission[np.asarray(traced)[blocked]] = records["transmission"][blocked]
+        for g, value, index in zip(traced, records["occlusion"].tolist(), records["occlusion_surface"].tolist()):
+            occlusion[g] = value
+            surface[g] = names[index] if index >= 0 else None
+    attenuations = [1.0 / max(d, config.min_distance_m) for d in distances]
+    air = np.asarray([[math.exp(-a * d) for a in bands.AIR_ABSORPTION_NP_PER_M] for d in distances]).reshape(N, 6)
+    opened = np.asarray(occlusion).reshape(N, 1)
+    level = np.asarray(gains, dtype=float).reshape(N, 1) * np.asarray(attenuations, dtype=float).reshape(N, 1)
+    band_gains = (level * air * (opened + (1.0 - opened) * transmission)).tolist()
+    return [{
+        "distance_m": distances[g],
+        "delay_s": distances[g] / config.c,
+        "distance_attenuation": attenuations[g],
+        "air_absorption": air[g].copy(),
+        "occlusion": occlusion[g],
+        "transmission": transmission[g].copy(),
+        "occlusion_surface": surface[g],
+        "source_directivity_gain": gains[g],
+        "band_gains": dict(zip(bands.FREQUENCY_BANDS, band_gains[g])),
+    } for g in range(N)]
 
 
 def simulate_direct(scene: Any, source: np.ndarray, listener: np.ndarray, config: Any,

@@ -10,6 +10,7 @@ import ctypes
 import math
 from collections import OrderedDict
 from dataclasses import dataclass, field
+from functools import lru_cache
 from threading import Lock
 from typing import Any, Mapping, Sequence
 
@@ -905,13 +906,19 @@ def read_bandwidth_gbs(device: torch.device, nbytes: int, *, repeats: int = 10, 
     return (buf.numel() // 4) * 16 * repeats * launches / (start.elapsed_time(stop) / 1000.0) / 1e9
 
 
-def device_info(device: int = 0) -> dict[str, Any]:
+@lru_cache(maxsize=None)
+def _device_info(device: int) -> tuple[str, str, int]:
+    """Name, compute capability and SM count of a device: the driver takes 2.5-3.5 ms to report its properties."""
     name = ctypes.create_string_buffer(256)
     major, minor, sms = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_int32()
-    _lib.check(_lib.load().ac_device_info(int(device), name, 256, ctypes.byref(major), ctypes.byref(minor),
+    _lib.check(_lib.load().ac_device_info(device, name, 256, ctypes.byref(major), ctypes.byref(minor),
                                           ctypes.byref(sms)), "ac_device_info")
-    return {"id": int(device), "name": name.value.decode(), "compute_capability": f"{major.value}.{minor.value}",
-            "sm_count": int(sms.value)}
+    return name.value.decode(), f"{major.value}.{minor.value}", int(sms.value)
+
+
+def device_info(device: int = 0) -> dict[str, Any]:
+    name, capability, sms = _device_info(int(device))
+    return {"id": int(device), "name": name, "compute_capability": capability, "sm_count": sms}
 
 
 def ray_bounce_count(buffers: TraceBuffers) -> int:
