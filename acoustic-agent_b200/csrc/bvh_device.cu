@@ -24,8 +24,8 @@
 // finds the node's median (k = n/2) and surfaces are scattered to the two
 // halves.  Steps are separated by a grid barrier whose waits are bounded.
 // Each remaining subtree of at most 1,024 or 2,048 surfaces is built by one CTA in
-// shared memory: per level, a bitonic sort of all its surfaces by (segment,
-// composite key) and a split of every internal segment at its half.  Surface
+// shared memory: per level, a bitonic sort of every node's surfaces by their ranks
+// on its axes and a split of every internal node at its half.  Surface
 // bounds are read once, at the leaves; every inner node's bounds are the union
 // of its children's, filled deepest level first (min and max do not depend on
 // the order they are taken in).
@@ -46,15 +46,15 @@
 
 namespace acbvh {
 
-// Surfaces per shared-memory subtree: 1024 (four CTAs per SM) for scenes of 2,049 to 2^18 - 1 surfaces, where the
-// extra cooperative level costs less than the larger subtrees' sorts; 2048 (two CTAs per SM) otherwise.
+// Surfaces per shared-memory subtree (two CTAs per SM): 1024 for scenes of 2,049 to 2^18 - 1 surfaces, where the extra
+// cooperative level costs less than the larger subtrees' sorts, and for scenes of no more than that, whose single CTA
+// is faster with two places per thread than with four (300 surfaces 0.18 ms against 0.23); 2048 otherwise.
 constexpr int kSmallMax = 2048;
 constexpr int kSmallMid = 1024;
 constexpr int64_t kSmallMidBelow = int64_t{1} << 18;
 constexpr int kChunk = 1024;           // surfaces per block work item in the large-node levels
 constexpr int kTopThreads = 256;
 constexpr int kItems = kChunk / kTopThreads;   // surfaces per thread in a chunk's scatter
-constexpr int kSmallThreads = 512;
 constexpr int kMaxPasses = 28;         // 3 centroid words x 8 digits + 4 index digits
 constexpr long long kSpinLimit = 1ll << 23;
 constexpr unsigned long long kSign = 0x8000000000000000ull;
@@ -529,66 +529,160 @@ __global__ void __launch_bounds__(kTopThreads) bvh_top_kernel(TopArgs A) {
 }
 
 // ------------------------------------------------------- small subtrees ----
+//
+// One CTA builds a subtree of n surfaces in shared memory.  Every comparison of the build is settled once, up front:
+// the surfaces are sorted by index (a surface's slot is its place in that order) and, per axis, by centroid key; a
+// slot's rank on an axis is the first place of its key in that order, so that equal keys have equal ranks.  A node's
+// order (its axes' keys, most recent axis first, then the surface index) is then one 44-bit word per surface: three
+// ranks and the slot.
+//
+// Level by level the words of every node are sorted.  A node of a level of blocks of s places holds at most s surfaces
+// and owns block b, from place b * s: its left half stays, its right half moves to the block's middle, so all sorts of
+// a level are one bitonic sort of aligned blocks, half as long as the last level's.  Each thread keeps two or four
+// neighbouring places in registers: short strides run in the thread, those within a warp's places by shuffles, longer
+// ones through shared memory.
+//
+// What bounds it is instruction issue: some 45,000 instructions per warp of 2,048 surfaces, a third of them in the three
+// sorts of 64-bit keys.  Comparing by slot through shared memory at every step of every level, the kernel was bound by
+// that memory's pipe (124 M bank conflicts at 2^20 surfaces; now 18 M).  Measured, whole builds: 2^20 warehouse
+// 3.64 -> 3.21 ms (this kernel 1.21 -> 0.79), 2^20 random 2.57 -> 2.25, 2^16 random 0.54 -> 0.51, one CTA with 2,000 /
+// 300 / 50 surfaces 0.45 / 0.21 / 0.133 -> 0.34 / 0.18 / 0.134.  Four places per thread at 1,024 surfaces too were
+// slower (2^16 0.56, 300 surfaces 0.23 ms: half the warps to hide latencies with).
 
-struct Entry {
-    uint16_t start, count;
+constexpr int kSmallThreads = 512;
+constexpr int kMaxSubtreeLevels = 32;
+constexpr unsigned kNoEntry = 0xFFFFu;
+constexpr unsigned long long kPadWord = ~0ull;   // sorts behind every word and key
+
+struct Entry {   // an internal node of the subtree
     int32_t node;
-    uint32_t chain;
+    uint16_t start, count;   // its surfaces' first place in the subtree's output, and their number
 };
 
-constexpr int kMaxSubtreeLevels = 32;
-
-// Shared-memory state of one subtree of at most N surfaces (N a power of two, at most 4096).
+// Shared-memory state of one subtree of at most N surfaces (N a power of two, at most 2048: ranks have 11 bits).
 template <int N>
 struct SmallSmem {
     static constexpr int kCapacity = N;
-    unsigned long long key[3][N];
-    int32_t gidx[N];
-    uint16_t lp[N];        // position -> slot, sorted every level
-    uint16_t segslot[N];   // slot -> start of its segment (0xFFFF: padding)
-    uint16_t cnt_at[N];    // segment start -> count
-    uint8_t chain_at[N];   // segment start -> axis order
-    uint8_t split_at[N];   // segment start -> depth at which it was split
-    Entry inner[N];        // every internal node of the subtree, level after level (at most n - 1)
-    unsigned long long part[kSmallThreads / 32][6];
+    static constexpr int kItems = N / kSmallThreads;   // places per thread
+    unsigned long long key[3][N];        // each axis's centroid keys, ascending
+    union {
+        unsigned long long word[N];      // items on their way between warps, in a sort of 64-bit words
+        struct {
+            unsigned word32[N];          // the same, in a level's sort
+            uint16_t lp[2][N];           // place -> slot, of this level / of the next one
+        };
+    };
+    Entry inner[N];                      // every internal node of the subtree, level after level (at most n - 1)
+    int32_t gidx[N];                     // slot -> surface, ascending
+    uint16_t rank[3][N];                 // slot -> rank of its key
+    uint16_t place[N];                   // internal node -> its block and (low 6 bits) its axis order
+    uint16_t node_at[2][N / 2];          // block -> internal node of this level / of the next one
+    unsigned part[kSmallThreads / 32][3];
+    LevelTab tab[2];                     // subtree sizes at this level's depth / at the next one's
     int level_begin[kMaxSubtreeLevels + 2];
     int nnext;
 };
 
-template <class M>
-__device__ __forceinline__ bool slot_less(const M &m, int a, int b) {
-    const unsigned sa = m.segslot[a], sb = m.segslot[b];
-    if (sa != sb) return sa < sb;
-    if (sa == 0xFFFFu) return a < b;
-    const uint32_t chain = m.chain_at[sa];
-    for (int j = 0; j < 3; ++j) {
-        const uint32_t axis = (chain >> (2 * j)) & 3u;
-        if (axis == 3u) break;
-        const unsigned long long ka = m.key[axis][a], kb = m.key[axis][b];
-        if (ka != kb) return ka < kb;
+// Sorts every aligned block of `s` places (a power of two) of the first `places` (another, s at least) in ascending
+// order of `v`; `w` moves along with its item.  Equal keys keep their places or swap: callers give such items no order.
+// A warp of nothing but padding has nothing to sort; in blocks of more than a warp's places the warps below `places`
+// wait for one another at a barrier of their own.
+template <bool kPayload, int IT, class K>
+__device__ __forceinline__ void sort_blocks(K (&v)[IT], unsigned (&w)[IT], int s, int places, K *word) {
+    constexpr int T = kSmallThreads;
+    const int tid = threadIdx.x;
+    if (s > 32 * IT) {
+        if ((tid & ~31) * IT >= places) return;
+    } else {
+        bool item = false;
+#pragma unroll
+        for (int u = 0; u < IT; ++u) item = item || v[u] != static_cast<K>(kPadWord);
+        if (!__any_sync(0xffffffffu, item)) return;
     }
-    return m.gidx[a] < m.gidx[b];
+    auto meet = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(places / IT) : "memory"); };
+    auto compare = [&](int u, int x, bool up) {   // places u < x of this thread
+        if (up ? v[x] < v[u] : v[u] < v[x]) {
+            const K k = v[u]; v[u] = v[x]; v[x] = k;
+            if (kPayload) { const unsigned p = w[u]; w[u] = w[x]; w[x] = p; }
+        }
+    };
+#pragma unroll 1
+    for (int k = 2; k <= s; k <<= 1) {
+#pragma unroll 1
+        for (int j = k >> 1; j >= IT; j >>= 1) {
+            const int d = j / IT;
+            const bool up = k == s || (tid & (k / IT)) == 0, keep_min = up == ((tid & d) == 0);
+            K ov[IT];
+            unsigned ow[IT];
+            if (d < 32) {
+#pragma unroll
+                for (int u = 0; u < IT; ++u) {
+                    ov[u] = __shfl_xor_sync(0xffffffffu, v[u], d);
+                    if (kPayload) ow[u] = __shfl_xor_sync(0xffffffffu, w[u], d);
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < IT; ++u) word[u * T + tid] = v[u];
+                meet();
+#pragma unroll
+                for (int u = 0; u < IT; ++u) ov[u] = word[u * T + (tid ^ d)];
+                meet();
+                if (kPayload) {
+#pragma unroll
+                    for (int u = 0; u < IT; ++u) word[u * T + tid] = w[u];
+                    meet();
+#pragma unroll
+                    for (int u = 0; u < IT; ++u) ow[u] = static_cast<unsigned>(word[u * T + (tid ^ d)]);
+                    meet();
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < IT; ++u)
+                if (keep_min ? ov[u] < v[u] : v[u] < ov[u]) {
+                    v[u] = ov[u];
+                    if (kPayload) w[u] = ow[u];
+                }
+        }
+#pragma unroll
+        for (int j = IT / 2; j > 0; j >>= 1) {
+            if (j >= k) continue;
+#pragma unroll
+            for (int u = 0; u < IT; ++u)
+                if ((u & j) == 0) compare(u, u | j, k == s || (k < IT ? (u & k) == 0 : (tid & (k / IT)) == 0));
+        }
+    }
 }
 
-// A leaf of the positions [s, s + c): its surfaces in ascending index order (bvh.py:48) and its bounds.
+// A leaf: the c surfaces of the places [p, p + c) in ascending index order (bvh.py:48) and their bounds; `s`: their
+// first place in the subtree's output.
 template <class M>
-__device__ void emit_leaf(M &m, const SmallArgs &A, const SmallRoot &r, int s, int c, int64_t node) {
-    for (int x = s + 1; x < s + c; ++x) {   // insertion sort of the leaf's slots by surface index
-        const uint16_t v = m.lp[x];
+__device__ void emit_leaf(M &m, uint16_t *lp, const SmallArgs &A, const SmallRoot &r, int p, int s, int c, int64_t node) {
+    for (int x = p + 1; x < p + c; ++x) {   // insertion sort of the leaf's slots, whose order is the surfaces'
+        const uint16_t v = lp[x];
         int y = x - 1;
-        while (y >= s && m.gidx[m.lp[y]] > m.gidx[v]) {
-            m.lp[y + 1] = m.lp[y];
+        while (y >= p && lp[y] > v) {
+            lp[y + 1] = lp[y];
             --y;
         }
-        m.lp[y + 1] = v;
+        lp[y + 1] = v;
     }
     unsigned long long mx[3] = {0ull, 0ull, 0ull}, mn_c[3] = {0ull, 0ull, 0ull};
-    for (int x = s; x < s + c; ++x) {
-        const int64_t g = m.gidx[m.lp[x]];
-        A.out_prims[r.start + x] = g;
+    for (int x = 0; x < c; x += 2) {   // two surfaces' loads in flight; an odd last one is read twice
+        const int64_t g0 = m.gidx[lp[p + x]], g1 = m.gidx[lp[p + min(x + 1, c - 1)]];
+        double h[6], l[6];
+#pragma unroll
         for (int a = 0; a < 3; ++a) {
-            mx[a] = max(mx[a], order_key(A.hi[3 * g + a]));
-            mn_c[a] = max(mn_c[a], ~order_key(A.lo[3 * g + a]));
+            h[a] = __ldg(A.hi + 3 * g0 + a);
+            l[a] = __ldg(A.lo + 3 * g0 + a);
+            h[3 + a] = __ldg(A.hi + 3 * g1 + a);
+            l[3 + a] = __ldg(A.lo + 3 * g1 + a);
+        }
+        A.out_prims[r.start + s + x] = g0;
+        if (x + 1 < c) A.out_prims[r.start + s + x + 1] = g1;
+#pragma unroll
+        for (int a = 0; a < 6; ++a) {
+            mx[a % 3] = max(mx[a % 3], order_key(h[a]));
+            mn_c[a % 3] = max(mn_c[a % 3], ~order_key(l[a]));
         }
     }
     for (int a = 0; a < 3; ++a) {
@@ -611,165 +705,224 @@ __device__ __forceinline__ void union_children(double *out_min, double *out_max,
     }
 }
 
-// Axis and key order of an internal node from its centroid key extents, and its record (bounds come later).
+// Rank extents of a node's surfaces, 16 bits each: maxima of the ranks and of their complements.
+struct Extents {
+    unsigned v[3];   // rank 0 | rank 1, rank 2 | ~rank 0, ~rank 1 | ~rank 2 (low | high half)
+    __device__ __forceinline__ void add(const Extents &o) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[c] = __vmaxu2(v[c], o.v[c]);
+    }
+};
+
+// Axis and key order of an internal node from its extents, and its record (bounds come later).
 template <class M>
-__device__ __forceinline__ void finish_inner(M &m, const SmallArgs &A, Entry &en, int depth,
-                                             const unsigned long long cmax[3], const unsigned long long cmin_c[3]) {
-    const uint32_t chain = push_axis(en.chain, widest_axis(cmax, cmin_c));
-    en.chain = chain;
-    m.chain_at[en.start] = static_cast<uint8_t>(chain);
-    m.cnt_at[en.start] = en.count;
-    m.split_at[en.start] = static_cast<uint8_t>(depth);
-    const int64_t node = en.node;
-    A.out_start[node] = -1;
-    A.out_count[node] = 0;
-    A.out_escape[node] = node + subtree_nodes(A.tab, depth, en.count);
+__device__ __forceinline__ void finish_inner(M &m, const SmallArgs &A, int x, int lev, const Extents &e) {
+    unsigned long long cmax[3], cmin_c[3];
+    const unsigned high[3] = {e.v[0] & 0xFFFFu, e.v[0] >> 16, e.v[1] & 0xFFFFu};
+    const unsigned low_c[3] = {e.v[1] >> 16, e.v[2] & 0xFFFFu, e.v[2] >> 16};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        cmax[a] = m.key[a][high[a]];
+        cmin_c[a] = ~m.key[a][0xFFFFu - low_c[a]];
+    }
+    const unsigned place = m.place[x];
+    m.place[x] = static_cast<uint16_t>((place & ~63u) | push_axis(place & 63u, widest_axis(cmax, cmin_c)));
+    const Entry en = m.inner[x];
+    A.out_start[en.node] = -1;
+    A.out_count[en.node] = 0;
+    A.out_escape[en.node] = en.node + subtree_nodes(m.tab, lev & 1, en.count);
 }
 
 // Internal nodes of a level number at most n / 2 (each holds two or more surfaces); all of them at most n - 1.
 template <class M>
-__device__ __forceinline__ void push_entry(M &m, int32_t *status, const Entry &e) {
+__device__ __forceinline__ void push_entry(M &m, int32_t *status, const Entry &e, int block, unsigned chain,
+                                           uint16_t *node_at) {
     const int at = atomicAdd(&m.nnext, 1);
-    if (at < M::kCapacity) m.inner[at] = e;
-    else atomicOr(status, AC_BVH_STATUS_INTERNAL);
+    if (at < M::kCapacity && block < M::kCapacity / 2) {
+        m.inner[at] = e;
+        m.place[at] = static_cast<uint16_t>((block << 6) | chain);
+        node_at[block] = static_cast<uint16_t>(at);
+    } else {
+        atomicOr(status, AC_BVH_STATUS_INTERNAL);
+    }
 }
 
 template <int N>
 __global__ void __launch_bounds__(kSmallThreads) bvh_small_kernel(SmallArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SmallSmem<N> &m = *reinterpret_cast<SmallSmem<N> *>(smem_raw);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int kWarps = kSmallThreads / 32;
+    constexpr int T = kSmallThreads, IT = SmallSmem<N>::kItems;
+    static_assert(IT == 2 || IT == 4, "two or four places per thread");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, first = tid * IT;
     if (ld_status(A.status) != 0) return;
     const SmallRoot r = A.roots[blockIdx.x];
     const int n = r.count;
-    int p2 = 1;
+    int p2 = 2;
     while (p2 < n) p2 <<= 1;
     const int32_t *src = r.buf ? A.perm1 : A.perm0;
-    for (int q = tid; q < N; q += kSmallThreads) {
-        m.chain_at[q] = static_cast<uint8_t>(kNoChain);
-        m.split_at[q] = 0xFF;
-        if (q < p2) {
-            m.lp[q] = static_cast<uint16_t>(q);
-            if (q < n) {
-                int32_t g = src[r.start + q];
-                if (bad_index(g, A.S, A.status)) g = 0;
-                m.gidx[q] = g;
-                for (int a = 0; a < 3; ++a) m.key[a][q] = A.ckey[a * A.S + g];
-                m.segslot[q] = 0;
-            } else {
-                m.segslot[q] = 0xFFFFu;
-            }
+
+    // slots: the surfaces in index order
+    unsigned long long v[IT];
+    unsigned w[IT] = {}, v32[IT];
+#pragma unroll
+    for (int u = 0; u < IT; ++u) {
+        v32[u] = static_cast<unsigned>(kPadWord);
+        if (first + u < n) {
+            const int32_t g = src[r.start + first + u];
+            v32[u] = bad_index(g, A.S, A.status) ? 0u : static_cast<unsigned>(g);
         }
     }
+    sort_blocks<false>(v32, w, p2, p2, m.word32);
+#pragma unroll
+    for (int u = 0; u < IT; ++u)
+        if (first + u < n) m.gidx[first + u] = static_cast<int32_t>(v32[u]);
+    // ranks: each axis's keys in ascending order
+#pragma unroll 1
+    for (int a = 0; a < 3; ++a) {
+#pragma unroll
+        for (int u = 0; u < IT; ++u) {
+            w[u] = static_cast<unsigned>(first + u);
+            v[u] = first + u < n ? A.ckey[a * A.S + m.gidx[first + u]] : kPadWord;
+        }
+        sort_blocks<true>(v, w, p2, p2, m.word);
+#pragma unroll
+        for (int u = 0; u < IT; ++u) m.key[a][first + u] = v[u];
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < IT; ++u) {
+            if (first + u >= n) continue;
+            int lo = first + u;
+            if (lo > 0 && m.key[a][lo - 1] == v[u]) {   // the first place of an equal key
+                int hi = lo;
+                lo = 0;
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (m.key[a][mid] < v[u]) lo = mid + 1; else hi = mid;
+                }
+            }
+            m.rank[a][w[u]] = static_cast<uint16_t>(lo);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < IT; ++u) m.lp[0][first + u] = static_cast<uint16_t>(first + u);
     __syncthreads();
     if (tid == 0) {
         const uint32_t parent_chain = r.parent >= 0 ? static_cast<uint32_t>(A.state[r.parent].chain) : kNoChain;
-        m.inner[0] = Entry{0, static_cast<uint16_t>(n), r.node, parent_chain};
+        m.inner[0] = Entry{r.node, 0, static_cast<uint16_t>(n)};
+        m.place[0] = static_cast<uint16_t>(parent_chain);
+        m.node_at[0][0] = n > A.leaf ? 0u : kNoEntry;
+        m.tab[0] = A.tab[r.depth];
         m.level_begin[0] = 0;
         m.level_begin[1] = n > A.leaf ? 1 : 0;
-        if (n <= A.leaf) emit_leaf(m, A, r, 0, n, r.node);
+        if (n <= A.leaf) emit_leaf(m, m.lp[0], A, r, 0, 0, n, r.node);
     }
     __syncthreads();
+
     int lev = 0;
     for (; lev < kMaxSubtreeLevels; ++lev) {
-        const int b = m.level_begin[lev], e = m.level_begin[lev + 1], ncur = e - b;
-        if (ncur <= 0) break;
-        const int depth = r.depth + lev;
-        // 1. centroid extents of every internal node: a thread per node, or warps per node while they are few
-        if (ncur >= kWarps) {
-            for (int x = b + tid; x < e; x += kSmallThreads) {
-                Entry &en = m.inner[x];
-                unsigned long long cmax[3] = {0ull, 0ull, 0ull}, cmin_c[3] = {0ull, 0ull, 0ull};
-                for (int q = en.start; q < en.start + en.count; ++q) {
-                    const int slot = m.lp[q];
-                    for (int a = 0; a < 3; ++a) {
-                        const unsigned long long k = m.key[a][slot];
-                        cmax[a] = max(cmax[a], k);
-                        cmin_c[a] = max(cmin_c[a], ~k);
-                    }
-                }
-                finish_inner(m, A, en, depth, cmax, cmin_c);
-            }
-        } else {
-            const int g = kWarps / ncur;
-            unsigned long long acc[6] = {0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
-            if (warp / g < ncur) {
-                const Entry en = m.inner[b + warp / g];
-                for (int q = en.start + (warp % g) * 32 + lane; q < en.start + en.count; q += g * 32) {
-                    const int slot = m.lp[q];
+        const int b = m.level_begin[lev], e = m.level_begin[lev + 1];
+        if (e <= b) break;
+        const int s = p2 >> lev, log_s = 31 - __clz(s);
+        const uint16_t *at = m.node_at[lev & 1];
+        uint16_t *next_at = m.node_at[(lev + 1) & 1];
+        if (s < 2) {   // cannot happen: a node of s places holds at most s surfaces
+            if (tid == 0) atomicOr(A.status, AC_BVH_STATUS_INTERNAL);
+            break;
+        }
+        if (tid == T - 1) m.tab[(lev + 1) & 1] = A.tab[r.depth + lev + 1];
+        // 1. this level's nodes, their surfaces and their extents
+        unsigned node[IT];
+        unsigned long long rk[IT];   // the ranks, 16 bits each
+        bool valid[IT];
+        Extents ext[IT];
 #pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        const unsigned long long k = m.key[a][slot];
-                        acc[a] = max(acc[a], k);
-                        acc[3 + a] = max(acc[3 + a], ~k);
-                    }
-                }
-            }
+        for (int u = 0; u < IT; ++u) {
+            const int q = first + u;
+            node[u] = q < p2 ? at[q >> log_s] : kNoEntry;
+            valid[u] = node[u] != kNoEntry && (q & (s - 1)) < m.inner[node[u]].count;
+            w[u] = valid[u] ? m.lp[lev & 1][q] : 0u;
+            const unsigned r0 = m.rank[0][w[u]], r1 = m.rank[1][w[u]], r2 = m.rank[2][w[u]];
+            rk[u] = r0 | (static_cast<unsigned long long>(r1) << 16) | (static_cast<unsigned long long>(r2) << 32);
+            ext[u].v[0] = valid[u] ? r0 | (r1 << 16) : 0u;
+            ext[u].v[1] = valid[u] ? r2 | ((0xFFFFu - r0) << 16) : 0u;
+            ext[u].v[2] = valid[u] ? (0xFFFFu - r1) | ((0xFFFFu - r2) << 16) : 0u;
+        }
 #pragma unroll
-            for (int j = 0; j < 6; ++j) {
-                unsigned long long v = acc[j];
-                for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-                if (lane == 0) m.part[warp][j] = v;
-            }
+        for (int u = 0; u < IT; u += 2) ext[u].add(ext[u + 1]);
+        if (IT == 4 && s >= 4) ext[0].add(ext[IT - 2]);
+        for (int d = 1; d < 32 && d * IT < s; d <<= 1) {
+            Extents o;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) o.v[c] = __shfl_xor_sync(0xffffffffu, ext[0].v[c], d);
+            ext[0].add(o);
+        }
+        if (s > 32 * IT) {
+            if (lane == 0)
+                for (int c = 0; c < 3; ++c) m.part[warp][c] = ext[0].v[c];
             __syncthreads();
-            if (tid < ncur) {
-                unsigned long long v[6];
-                for (int j = 0; j < 6; ++j) {
-                    v[j] = m.part[tid * g][j];
-                    for (int w = 1; w < g; ++w) v[j] = max(v[j], m.part[tid * g + w][j]);
-                }
-                finish_inner(m, A, m.inner[b + tid], depth, v, v + 3);
-            }
+            if ((first & (s - 1)) == 0 && node[0] != kNoEntry)
+                for (int x = 1; x < s / (32 * IT); ++x)
+                    ext[0].add(Extents{{m.part[warp + x][0], m.part[warp + x][1], m.part[warp + x][2]}});
         }
+        if ((first & (s - 1)) == 0 && node[0] != kNoEntry) finish_inner(m, A, node[0], lev, ext[0]);
+        if (IT == 4 && s == 2 && node[IT - 2] != kNoEntry) finish_inner(m, A, node[IT - 2], lev, ext[IT - 2]);
         if (tid == 0) m.nnext = e;
-        __syncthreads();
-        // 2. bitonic sort of all positions by (segment, key in the segment's axis order, surface index).
-        // Warp w owns pairs [w*ppw, (w+1)*ppw), i.e. positions [2*w*ppw, 2*(w+1)*ppw) while the stride j is at
-        // most ppw: such stages need only the warp's own barrier.
-        const int pairs = p2 >> 1;
-        const int ppw = max(1, pairs / kWarps);
-        for (int k = 2; k <= p2; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int rr = lane; rr < ppw; rr += 32) {
-                    const int i = warp * ppw + rr;
-                    if (i >= pairs) break;
-                    const int lo = ((i & ~(j - 1)) << 1) | (i & (j - 1));
-                    const int hi = lo | j;
-                    const int a = m.lp[lo], bb = m.lp[hi];
-                    const bool up = (lo & k) == 0;
-                    if (slot_less(m, bb, a) == up) {
-                        m.lp[lo] = static_cast<uint16_t>(bb);
-                        m.lp[hi] = static_cast<uint16_t>(a);
-                    }
+        if (s >= 4)
+            for (int x = tid; x < (p2 >> (log_s - 1)); x += T) next_at[x] = kNoEntry;
+        __syncthreads();   // the places are in registers, the axis orders written
+        // 2. the nodes' surfaces in order; 3. the left halves stay, the right halves move to the middle of their blocks
+        uint16_t *next_lp = m.lp[(lev + 1) & 1];
+        auto move = [&](int u, unsigned slot) {
+            const int k = (first + u) & (s - 1), half = m.inner[node[u]].count / 2;
+            next_lp[first + u - k + (k < half ? k : s / 2 + k - half)] = static_cast<uint16_t>(slot);
+        };
+        if (lev == 0) {   // the words of the node's own order
+#pragma unroll
+            for (int u = 0; u < IT; ++u) {
+                v[u] = kPadWord;
+                if (!valid[u]) continue;
+                const unsigned chain = m.place[node[u]] & 63u;
+                v[u] = w[u];
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    const unsigned axis = (chain >> (2 * j)) & 3u;
+                    if (axis != 3u) v[u] |= ((rk[u] >> (16 * axis)) & 0x7FFull) << (33 - 11 * j);
                 }
-                const int next_j = j > 1 ? j >> 1 : k;
-                const bool last = k == p2 && j == 1;
-                if (!last && j <= ppw && next_j <= ppw) __syncwarp();
-                else __syncthreads();
             }
-        }
-        // 3. the right halves of the split segments become segments of their own
-        for (int q = tid; q < n; q += kSmallThreads) {
-            const int slot = m.lp[q];
-            const unsigned s0 = m.segslot[slot];
-            if (m.split_at[s0] == static_cast<uint8_t>(depth)) {
-                const unsigned half = s0 + m.cnt_at[s0] / 2u;
-                if (static_cast<unsigned>(q) >= half) m.segslot[slot] = static_cast<uint16_t>(half);
+            sort_blocks<false>(v, w, s, p2, m.word);
+#pragma unroll
+            for (int u = 0; u < IT; ++u)
+                if (v[u] != kPadWord) move(u, static_cast<unsigned>(v[u]) & 0x7FFu);
+        } else {   // the surfaces lie in the parent's order: the rank on the new axis, then the place
+#pragma unroll
+            for (int u = 0; u < IT; ++u) {
+                v32[u] = static_cast<unsigned>(kPadWord);
+                if (!valid[u]) continue;
+                const unsigned axis = m.place[node[u]] & 3u;
+                v32[u] = (static_cast<unsigned>(rk[u] >> (16 * axis)) & 0x7FFu) << 11 | ((first + u) & (s - 1));
             }
+            sort_blocks<false>(v32, w, s, p2, m.word32);
+#pragma unroll
+            for (int u = 0; u < IT; ++u)
+                if (v32[u] != static_cast<unsigned>(kPadWord))
+                    move(u, m.lp[lev & 1][((first + u) & ~(s - 1)) + (v32[u] & 0x7FFu)]);
         }
         __syncthreads();
         // 4. children: leaves are written now, internal ones form the next level
-        for (int x = b + tid; x < e; x += kSmallThreads) {
+        for (int x = b + tid; x < e; x += T) {
             const Entry en = m.inner[x];
+            const unsigned chain = m.place[x] & 63u;
+            const int block = m.place[x] >> 6, p = block * s;
             const int lc = en.count / 2, rc = en.count - lc;
             const int64_t lnode = en.node + 1;
-            const int64_t rnode = lnode + subtree_nodes(A.tab, depth + 1, lc);
-            if (lc <= A.leaf) emit_leaf(m, A, r, en.start, lc, lnode);
-            else push_entry(m, A.status, Entry{en.start, static_cast<uint16_t>(lc), static_cast<int32_t>(lnode), en.chain});
-            if (rc <= A.leaf) emit_leaf(m, A, r, en.start + lc, rc, rnode);
-            else push_entry(m, A.status, Entry{static_cast<uint16_t>(en.start + lc), static_cast<uint16_t>(rc),
-                                               static_cast<int32_t>(rnode), en.chain});
+            const int64_t rnode = lnode + subtree_nodes(m.tab, (lev + 1) & 1, lc);
+            if (lc <= A.leaf) emit_leaf(m, next_lp, A, r, p, en.start, lc, lnode);
+            else push_entry(m, A.status, Entry{static_cast<int32_t>(lnode), en.start, static_cast<uint16_t>(lc)},
+                            2 * block, chain, next_at);
+            if (rc <= A.leaf) emit_leaf(m, next_lp, A, r, p + s / 2, en.start + lc, rc, rnode);
+            else push_entry(m, A.status, Entry{static_cast<int32_t>(rnode), static_cast<uint16_t>(en.start + lc),
+                                               static_cast<uint16_t>(rc)}, 2 * block + 1, chain, next_at);
         }
         __syncthreads();
         if (tid == 0) m.level_begin[lev + 2] = min(m.nnext, N);
@@ -779,7 +932,7 @@ __global__ void __launch_bounds__(kSmallThreads) bvh_small_kernel(SmallArgs A) {
     // 5. bounds of the internal nodes, deepest level first, from their children's
     for (int l = lev - 1; l >= 0; --l) {
         const int depth = r.depth + l;
-        for (int x = m.level_begin[l] + tid; x < m.level_begin[l + 1]; x += kSmallThreads) {
+        for (int x = m.level_begin[l] + tid; x < m.level_begin[l + 1]; x += T) {
             const Entry en = m.inner[x];
             const int64_t left = static_cast<int64_t>(en.node) + 1;
             union_children(A.out_min, A.out_max, en.node, left, left + subtree_nodes(A.tab, depth + 1, en.count / 2));
@@ -1056,7 +1209,7 @@ extern "C" int ac_bvh_build_device(const double *bounds_min, const double *bound
     }
     {
         static_assert(sizeof(SmallSmem<kSmallMax>) <= 227 * 1024, "subtree state must fit shared memory");
-        const bool mid = p.small_max == kSmallMid;
+        const bool mid = p.small_max == kSmallMid || S <= kSmallMid;
         const size_t smem = mid ? sizeof(SmallSmem<kSmallMid>) : sizeof(SmallSmem<kSmallMax>);
         AC_CUDA_TRY(cudaFuncSetAttribute(mid ? bvh_small_kernel<kSmallMid> : bvh_small_kernel<kSmallMax>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
