@@ -336,8 +336,8 @@ __device__ __forceinline__ int rec_tag(const T *rec) { return tag_bits(__ldg(rec
 //
 // What bounds it now is divergence: 3 of 32 lanes are active per instruction.  Measured with the rays of a small launch
 // spread over more warps (warp_lanes): furnished U room in BVH mode, 100 bounces, 500 / 5,000 / 20,000 / 100,000 rays
-// 6.36 / 6.25 / 7.01 / 17.1 -> 2.83 / 3.51 / 5.69 / 11.5 ms; apartment, 2,000 / 20,000 rays 11.6 / 12.7 -> 5.06 / 8.2;
-// shoebox, linear, 50 bounces, 500 / 5,000 / 20,000 rays 0.69 / 0.71 / 1.01 -> 0.56 / 0.71 / 1.02.
+// 6.36 / 6.25 / 7.01 / 17.1 -> 2.07 / 3.5 / 5.5 / 11.1 ms; apartment, 2,000 / 20,000 rays 11.6 / 12.7 -> 4.1 / 8.3;
+// shoebox, linear, 50 bounces, 500 / 5,000 / 20,000 rays 0.69 / 0.71 / 1.01 -> 0.44 / 0.68 / 1.03.
 
 __device__ __forceinline__ double approx_inverse(double x) {   // |x| between 1e-30 and 1e30
     return static_cast<double>(__frcp_rn(static_cast<float>(x)));

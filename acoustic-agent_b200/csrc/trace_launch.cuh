@@ -20,8 +20,9 @@ constexpr int kDefaultBlock = 256;
 // falls with the lanes it carries (its queries end with the slowest lane's), so its rays are spread over up to two
 // warps per scheduler (furnished U room, 100 bounces: 2,000 rays 0.98 -> 0.77 ms, 10,000 rays 1.06 -> 0.88; with three
 // warps 0.92, and 30,000 rays get slower).  Fewer lanes than `least` gain nothing: 4 where the rays of a warp descend a
-// BVH on their own (float64 too: 5,000 rays 3.5 ms, with 2 lanes or 16 warps per SM no better, full warps 5.6), 16 in
-// the lockstep scan (shoebox, 10,000 rays 0.36 -> 0.33 ms; 0.35 with 8).
+// BVH on their own, 16 in the lockstep scan (shoebox, 10,000 rays 0.36 -> 0.33 ms; 0.35 with 8).  The float64 walks are
+// so much longer than what their lanes share that a warp per ray pays: with at least 1 / 2 / 4 / 8 / 32 lanes, U room,
+// 500 rays 2.07 / 2.40 / 2.83 / 3.30 / 5.08 ms, shoebox, 500 rays 0.44 / 0.49 / 0.53 / 0.58 / 0.67.
 inline int warp_lanes(int device, int64_t rays, int least) {
     const int64_t warps = static_cast<int64_t>(device_sm_count(device)) * 8;
     return static_cast<int>(std::min<int64_t>(32, std::max<int64_t>(least, (rays + warps - 1) / warps)));
@@ -213,7 +214,7 @@ inline int launch_single(const ac_scene_s *scene, const ac_trace_params *p, cons
     if (block % 32 != 0 || block > 256) return fail(AC_ERR_INVALID, "block_size must be a multiple of 32 up to 256");
     if (p->num_rays > 0) {
         BatchTable none{};
-        none.lanes = p->grid_blocks > 0 ? 32 : warp_lanes(scene->device, p->num_rays, 4);
+        none.lanes = p->grid_blocks > 0 ? 32 : warp_lanes(scene->device, p->num_rays, 1);
         const int grid = persistent_grid<T, true>(scene->device, block, spread_rays(p->num_rays, none.lanes), p->grid_blocks);
         trace_kernel<T, true><<<grid, block, 0, stream>>>(job, none);
         AC_CUDA_TRY(cudaGetLastError());
@@ -339,7 +340,7 @@ inline int launch_batch(const ac_job *jobs_in, const int32_t *indices, int32_t c
         table.num_jobs = count;
         table.total_rays = total;
         table.work_counter = counter;
-        table.lanes = cfg && cfg->grid_blocks > 0 ? 32 : warp_lanes(device, total, 4);
+        table.lanes = cfg && cfg->grid_blocks > 0 ? 32 : warp_lanes(device, total, 1);
         const int grid = persistent_grid<T, false>(device, block, spread_rays(total, table.lanes), cfg ? cfg->grid_blocks : 0);
         Job<T> unused;
         std::memset(&unused, 0, sizeof(unused));
