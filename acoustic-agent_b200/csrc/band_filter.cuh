@@ -39,6 +39,7 @@
 #include <type_traits>
 
 #include "common.h"
+#include "filter_steps.h"
 
 namespace ac {
 namespace {
@@ -110,7 +111,7 @@ __device__ __forceinline__ void filter_block(const FilterSignal *signals, Filter
     int longest = 0;
 #pragma unroll
     for (int j = 0; j < kSignals; ++j) longest = max(longest, signals[j].n_len);
-    const int blocks = (longest + kStep - 1) / kStep;
+    const int blocks = filter_steps(longest, kStep);
     {   // the history before the first sample is +0.0
         unsigned *words = reinterpret_cast<unsigned *>(&m);
         for (int i = threadIdx.x; i < static_cast<int>(sizeof(m) / 4); i += Shape::kThreads) words[i] = 0u;
@@ -121,10 +122,11 @@ __device__ __forceinline__ void filter_block(const FilterSignal *signals, Filter
     auto load = [&](int k) {   // loader warp: step k's samples, lane = sample
 #pragma unroll
         for (int jh = 0; jh < kSignals * (kStep / 32); ++jh) {
-            const int j = jh / (kStep / 32), n = k * kStep + jh % (kStep / 32) * 32 + lane;
+            const int j = jh / (kStep / 32);
+            const unsigned n = filter_sample(k, kStep, jh % (kStep / 32) * 32 + lane);
             const FilterSignal sg = signals[j];
-            const bool valid = n < sg.n_len;
-            const double *p = sg.x + (valid ? n : 0);
+            const bool valid = in_signal(n, sg.n_len);
+            const double *p = sg.x + (valid ? n : 0u);
 #pragma unroll
             for (int b = 0; b < kInputs; ++b)
                 cp_async8_zfill(&m.x[n & (kRows - 1)][j * kInputs + b], p + b * sg.band_stride, valid);
@@ -155,7 +157,7 @@ __device__ __forceinline__ void filter_block(const FilterSignal *signals, Filter
             const int k = i - 1 - 2 * s;
             if (k >= 0 && k < blocks && has_chain) {
                 const double *vp = &m.v[s][k & 1][0][lane];
-                float *yp = &m.y[s][(k * kStep) & (kRows - 1)][lane];
+                float *yp = &m.y[s][filter_sample(k, kStep, 0) & (kRows - 1)][lane];
                 double v[8], next[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) v[u] = vp[u * kLanes];
@@ -191,7 +193,7 @@ __device__ __forceinline__ void filter_block(const FilterSignal *signals, Filter
         for (int i = 0; i < steps; ++i) {
             const int k = i - 2 * s;
             if (k >= 0 && k < blocks && has_chain) {
-                const int n = k * kStep + first;
+                const unsigned n = filter_sample(k, kStep, first);
                 double *vp = &m.v[s][k & 1][first][slot];
                 double x[kRun + 2];   // x[u + 2]: sample n + u
                 if (s == 0) {
@@ -228,9 +230,10 @@ __device__ __forceinline__ void filter_block(const FilterSignal *signals, Filter
             if (k >= 0) {
 #pragma unroll
                 for (int jh = 0; jh < kSignals * (kStep / 32); ++jh) {
-                    const int j = jh / (kStep / 32), n = k * kStep + jh % (kStep / 32) * 32 + lane;
+                    const int j = jh / (kStep / 32);
+                    const unsigned n = filter_sample(k, kStep, jh % (kStep / 32) * 32 + lane);
                     const FilterSignal sg = signals[j];
-                    if (n < sg.n_len) {
+                    if (in_signal(n, sg.n_len)) {
                         const double x5 = __ldg(sg.x + 5 * sg.band_stride + n);
                         const float *y = &m.y[kSections - 1][n & (kRows - 1)][j * kChains];
                         const float *lower = kShared ? y : y + 5;   // lower[b - 1]: band b's lower low-pass
