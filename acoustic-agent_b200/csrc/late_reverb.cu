@@ -17,7 +17,8 @@
 //       memory to the next (Biquad::run);
 //   warp 3: the six sections of the output cascade, a lane each;
 //   warp 4: the Hadamard mix and the delay lines' new samples (global memory,
-//       L2-resident, coalesced per line), lane i taking sample i of the step;
+//       L2-resident, coalesced per line), lane i taking sample i of the step
+//       (in short steps two lanes a sample, eight lines each);
 //   warp 5: the sum of the line outputs and the four all-pass stages (their
 //       delays are S or more, so a step's samples are independent);
 //   warp 6: the delay lines' next samples;
@@ -29,9 +30,12 @@
 // 2.47 ms (43 cycles per sample) against 4.3 ms (76) with shuffles between the
 // bands of a line in every sample and a barrier every 32; 256 of 30,000 samples
 // (16 kHz, S = 32, two blocks per SM) 1.35 ms against 1.94, 1,184 of them 6.1
-// against 8.1, where the shared-memory pipe is 66 % busy.  Input parts on warps of their own, as in
-// band_filter.cuh, took 44 cycles: they double the shared-memory traffic, which
-// with 96 sections is then what bounds the step.
+// against 8.1, where the shared-memory pipe is 66 % busy.  In short steps what
+// bounds it is the mix and the loads, some 700 cycles whatever the step: one
+// impulse of 16,000 samples with delays from 144 takes 0.525 ms (S = 16, 64
+// cycles per sample), from 128 0.575 (S = 14, 71), against 0.648.  Input parts
+// on warps of their own, as in band_filter.cuh, took 44 cycles: they double the
+// shared-memory traffic, which with 96 sections is then what bounds the step.
 //
 // ac_late_tail restates the rest of _render_parametric_fdn_late_reverb
 // (:2588-2640): bandlimit_band_signals of the impulse (the crossover filter
@@ -94,6 +98,10 @@ constexpr int kFdnThreads = 256;
 // What a sample computes reaches the delay lines in the sixth step after its first section's, and the lines are read
 // two steps ahead: the pipeline needs delays of at least kFdnLatency * S samples.
 constexpr int kFdnLatency = 9;
+// Lanes that share a sample's sixteen lines in the mix and in the loads of the delay lines: with steps of 16 samples or
+// fewer two of them take eight lines each (one impulse in steps of 16: 0.525 ms against 0.588, 444 of them 1.35 against
+// 1.66).
+constexpr int fdn_lanes_per_sample(int step) { return step <= 16 ? 2 : 1; }
 
 // One absorptive or tone section (steam_rt.py:2261-2275, :2312-2325) of one lane, in float64:
 //     y0 = b0*x0 + b1*x1 + b2*x2 - a1*y1 - a2*y2, left to right.
@@ -124,7 +132,7 @@ struct Biquad {
     // S samples from column xp to column yp of rows kPitch apart.
     template <int S, int kPitch>
     __device__ __forceinline__ void run(const double *xp, double *yp) {
-        constexpr int kAhead = 4;
+        constexpr int kAhead = S % 4 == 0 ? 4 : 2;
         static_assert(S % kAhead == 0, "whole groups");
         double v[kAhead], x[kAhead];
 #pragma unroll
@@ -177,10 +185,13 @@ __global__ void __launch_bounds__(kFdnThreads, 2) fdn_kernel(const FdnJobDev *jo
         __syncwarp();
         asm volatile("bar.sync 1, %0;" ::"n"(kFdnThreads) : "memory");
     };
-    // lane's sample (pass h) of line l in the step that `table` stands at; advance() moves it one step on
-    auto offset_of = [&](const FdnLine *table, int l, int h) {
+    // the lines of this lane in the mix and the loads, and its sample of a pass
+    constexpr int kShare = kLines / fdn_lanes_per_sample(S), kSamples = 32 / fdn_lanes_per_sample(S);
+    const int own = lane % kSamples, first_line = lane / kSamples * kShare;
+    // sample r of line l in the step that `table` stands at; advance() moves it one step on
+    auto offset_of = [&](const FdnLine *table, int l, int r) {
         const FdnLine line = table[l];
-        const int p = line.pos + 32 * h + lane;
+        const int p = line.pos + r;
         return line.start + (p >= line.delay ? p - line.delay : p);
     };
     auto advance = [&](FdnLine *table) {
@@ -224,27 +235,37 @@ __global__ void __launch_bounds__(kFdnThreads, 2) fdn_kernel(const FdnJobDev *jo
             if (k >= 0 && k < blocks) {
 #pragma unroll 1
                 for (int h = 0; h < kPasses; ++h) {
-                    const int r = 32 * h + lane;
+                    const int r = 32 * h + own;
+                    double d[kShare] = {};
+                    int offset[kShare];   // all addresses before the first store, which a later load would wait for
                     if (r < S) {
-                        int offset[kLines];   // all addresses before the first store, which a later load would wait for
 #pragma unroll
-                        for (int l = 0; l < kLines; ++l) offset[l] = offset_of(m.mix_line, l, h);
-                        const double *row = &m.y[k & 1][r][kBandSections * kLines];
-                        double d[kLines];
+                        for (int l = 0; l < kShare; ++l) offset[l] = offset_of(m.mix_line, first_line + l, r);
+                        const double *row = &m.y[k & 1][r][kBandSections * kLines + first_line];
 #pragma unroll
-                        for (int l = 0; l < kLines; ++l) d[l] = row[l];
+                        for (int l = 0; l < kShare; ++l) d[l] = row[l];
 #pragma unroll
-                        for (int stride = 1; stride < kLines; stride *= 2)
+                        for (int stride = 1; stride < kShare; stride *= 2)
 #pragma unroll
-                            for (int a = 0; a < kLines; ++a)
+                            for (int a = 0; a < kShare; ++a)
                                 if ((a & stride) == 0) {
                                     const double one = d[a], two = d[a + stride];
                                     d[a] = one + two;
                                     d[a + stride] = one - two;
                                 }
+                    }
+                    if constexpr (kShare < kLines) {   // the last stride, between the two lanes of a sample
+                        static_assert(kShare * 2 == kLines, "two lanes per sample");
+#pragma unroll
+                        for (int l = 0; l < kShare; ++l) {
+                            const double other = __shfl_xor_sync(0xffffffffu, d[l], kSamples);
+                            d[l] = first_line == 0 ? d[l] + other : other - d[l];
+                        }
+                    }
+                    if (r < S) {
                         const double injection = k == 0 && r == 0 ? 1.0 : 0.0;
 #pragma unroll
-                        for (int l = 0; l < kLines; ++l) lines[offset[l]] = injection + 0.25 * d[l];
+                        for (int l = 0; l < kShare; ++l) lines[offset[l]] = injection + 0.25 * d[l];
                     }
                 }
                 advance(m.mix_line);
@@ -302,23 +323,33 @@ __global__ void __launch_bounds__(kFdnThreads, 2) fdn_kernel(const FdnJobDev *jo
             barrier();
         }
     } else if (warp == 6) {
-        // the delay lines' samples, a sample per lane, read two steps ahead (around L1: the mix writes them) and
-        // stored to the next step's buffer; sample n of a line is at n mod delay
-        double x[kPasses][kLines];
+        // the delay lines' samples, read two steps ahead (around L1: the mix writes them) and stored to the next step's
+        // buffer; sample n of a line is at n mod delay
+        double x[kPasses][kShare];
+        // one branch around a pass's loads: with a condition per load they followed one another
         auto fetch = [&] {
 #pragma unroll
-            for (int h = 0; h < kPasses; ++h)
+            for (int h = 0; h < kPasses; ++h) {
+                const int r = 32 * h + own;
+                if (r < S) {
+                    int offset[kShare];
 #pragma unroll
-                for (int l = 0; l < kLines; ++l)
-                    x[h][l] = 32 * h + lane < S ? __ldcg(lines + offset_of(m.load_line, l, h)) : 0.0;
+                    for (int l = 0; l < kShare; ++l) offset[l] = offset_of(m.load_line, first_line + l, r);
+#pragma unroll
+                    for (int l = 0; l < kShare; ++l) x[h][l] = __ldcg(lines + offset[l]);
+                }
+            }
             advance(m.load_line);
         };
         auto store = [&](int k) {
 #pragma unroll
-            for (int h = 0; h < kPasses; ++h)
+            for (int h = 0; h < kPasses; ++h) {
+                const int r = 32 * h + own;
+                if (r < S) {
 #pragma unroll
-                for (int l = 0; l < kLines; ++l)
-                    if (32 * h + lane < S) m.y[k & 1][32 * h + lane][l] = x[h][l];
+                    for (int l = 0; l < kShare; ++l) m.y[k & 1][r][first_line + l] = x[h][l];
+                }
+            }
         };
         fetch();
         store(0);
@@ -596,8 +627,11 @@ constexpr int kMaxSmem = 227 * 1024;
 // all-pass samples are independent within a step and whose buffers fit shared memory.  A larger step has fewer barriers
 // per sample, but a step of 64 takes a whole SM (135 KB), so beyond one impulse per SM a step of 32, two blocks per SM,
 // is faster (296 impulses of 48 kHz: 72 cycles per sample against two waves of 47).  A step of 40 would fit the designs
-// of 16 kHz, but its mix takes two passes of 32 lanes and it is no faster (54 cycles against 47).  The reference's designs have delays of at least 841 samples from 32 kHz up, 361 at 16 kHz and 289 from
-// 7 kHz; a step of 8 meets every accepted delay.
+// of 16 kHz, but its mix takes two passes of 32 lanes and it is no faster (54 cycles against 47).  The reference's
+// designs have delays of at least 841 samples from 32 kHz up, 361 at 16 kHz, 289 from 7 kHz and 169 at 4.5 kHz; a step of
+// 14 meets every accepted delay.  1 / 444 impulses of 16,000 samples, shortest delay 128: 0.575 / 1.39 ms with 14, 0.67 /
+// 1.49 with 12, 1.62 / 3.87 with 8, 0.65 / 1.76 with the shuffles and a barrier every 32 samples; delay 144 with a step
+// of 16: 0.525 / 1.35.
 int fdn_step(const FdnLayout &l, int num_jobs, int sms) {
     const size_t ap = static_cast<size_t>(l.max_allpass_doubles) * sizeof(double);
     auto fits = [&](int step, size_t smem) {
@@ -605,10 +639,11 @@ int fdn_step(const FdnLayout &l, int num_jobs, int sms) {
     };
     if (num_jobs <= sms && fits(64, sizeof(FdnSmem<64>))) return 64;
     if (fits(32, sizeof(FdnSmem<32>))) return 32;
-    return 8;
+    if (fits(16, sizeof(FdnSmem<16>))) return 16;
+    return 14;
 }
-static_assert(kFdnLatency * 8 <= AC_FDN_MIN_DELAY && 8 <= kMinAllpass, "a step of 8 meets every accepted design");
-static_assert(sizeof(FdnSmem<8>) + AC_FDN_ALLPASS * AC_FDN_MAX_ALLPASS * sizeof(double) <= kMaxSmem, "and fits");
+static_assert(kFdnLatency * 14 <= AC_FDN_MIN_DELAY && 14 <= kMinAllpass, "a step of 14 meets every accepted design");
+static_assert(sizeof(FdnSmem<14>) + AC_FDN_ALLPASS * AC_FDN_MAX_ALLPASS * sizeof(double) <= kMaxSmem, "and fits");
 
 template <int S>
 int launch_fdn(const FdnJobDev *jobs, int num_jobs, double *pool, int max_allpass_doubles, cudaStream_t stream) {
@@ -726,7 +761,8 @@ extern "C" int ac_fdn_impulse(const ac_fdn_job *jobs, int32_t num_jobs, void *wo
     switch (ac::fdn_step(l, num_jobs, sms)) {
         case 64: return ac::launch_fdn<64>(d_jobs, num_jobs, lines, l.max_allpass_doubles, stream);
         case 32: return ac::launch_fdn<32>(d_jobs, num_jobs, lines, l.max_allpass_doubles, stream);
-        default: return ac::launch_fdn<8>(d_jobs, num_jobs, lines, l.max_allpass_doubles, stream);
+        case 16: return ac::launch_fdn<16>(d_jobs, num_jobs, lines, l.max_allpass_doubles, stream);
+        default: return ac::launch_fdn<14>(d_jobs, num_jobs, lines, l.max_allpass_doubles, stream);
     }
 }
 
