@@ -118,26 +118,28 @@ __global__ void finalize_f32_kernel(const Job<float> *jobs, const FinalizeTarget
 
 using FastKernel = void (*)(const Job<float>, const FastScene, const FastTable);
 
-template <bool kSingle, bool kVisual, bool kShards, bool kLean>
+template <bool kSingle, bool kVisual, bool kOwnSums, bool kLean>
 FastKernel pick_stream(bool philox, bool amb) {
     if (philox)
-        return amb ? trace_fast_kernel<kSingle, true, true, kVisual, false, kShards, kLean>
-                   : trace_fast_kernel<kSingle, true, false, kVisual, false, kShards, kLean>;
-    return amb ? trace_fast_kernel<kSingle, false, true, kVisual, false, kShards, kLean>
-               : trace_fast_kernel<kSingle, false, false, kVisual, false, kShards, kLean>;
+        return amb ? trace_fast_kernel<kSingle, true, true, kVisual, false, kOwnSums, kLean>
+                   : trace_fast_kernel<kSingle, true, false, kVisual, false, kOwnSums, kLean>;
+    return amb ? trace_fast_kernel<kSingle, false, true, kVisual, false, kOwnSums, kLean>
+               : trace_fast_kernel<kSingle, false, false, kVisual, false, kOwnSums, kLean>;
 }
 
 template <bool kSingle, bool kLean>
-FastKernel pick_variant(bool philox, bool amb, bool visual, bool shards) {
-    if (visual) return pick_stream<kSingle, true, false, kLean>(philox, amb);
-    return !kSingle && shards ? pick_stream<kSingle, false, !kSingle, kLean>(philox, amb)
-                              : pick_stream<kSingle, false, false, kLean>(philox, amb);
+FastKernel pick_variant(bool philox, bool amb, bool visual, bool own_sums) {
+    if (visual)   // batches with visual candidates have no copies
+        return kSingle && own_sums ? pick_stream<kSingle, true, kSingle, kLean>(philox, amb)
+                                   : pick_stream<kSingle, true, false, kLean>(philox, amb);
+    return own_sums ? pick_stream<kSingle, false, true, kLean>(philox, amb)
+                    : pick_stream<kSingle, false, false, kLean>(philox, amb);
 }
 
 template <bool kSingle>
-FastKernel pick_kernel(bool philox, bool amb, bool visual, bool shards, bool lean) {
-    return lean ? pick_variant<kSingle, true>(philox, amb, visual, shards)
-                : pick_variant<kSingle, false>(philox, amb, visual, shards);
+FastKernel pick_kernel(bool philox, bool amb, bool visual, bool own_sums, bool lean) {
+    return lean ? pick_variant<kSingle, true>(philox, amb, visual, own_sums)
+                : pick_variant<kSingle, false>(philox, amb, visual, own_sums);
 }
 
 // Whether the lean kernels can trace a scene: no boxes in the lockstep scan, no four-wide BVH.
@@ -257,27 +259,29 @@ int launch_trace_f32(const ac_scene_s *scene, const ac_trace_params *p, const ac
     table.lanes = p->grid_blocks > 0 ? 32 : warp_lanes(scene->device, p->num_rays, scene->fast.num_bvh_nodes > 0 ? 4 : 16);
     table.chunk_rays = std::min(kDefaultChunkRays, table.lanes);
     table.chunk_counter = reinterpret_cast<unsigned long long *>(o->counters) + 4;
-    table.stack_words = static_cast<int32_t>(stack_smem_bytes(entries) / sizeof(int));
+    const int64_t cells = static_cast<int64_t>(kBands) * p->num_bins * (job.ambisonic_fx ? 4 : 1) + scene->num_surfaces;
+    const int64_t sum_bytes = 4 * (4 * cells + 2 * scene->num_surfaces);
+    const bool own_sums = sum_bytes <= kSharedSumBytes;
+    // beside the sums no deeper stack than the tree uses, so that three blocks still fit an SM (U room, 400 bins, 100,000
+    // rays: 0.98 ms with two, 0.72 with three; what lies above the need is never read)
+    if (own_sums) entries = std::min(entries, static_cast<int>(scene->bvh_stack_need));
     const FastKernel kernel = pick_kernel<true>(p->rng_mode == AC_RNG_PHILOX, p->render_ambisonics != 0,
-                                                p->visual_limit > 0, false, scene_is_lean(scene->fast));
+                                                p->visual_limit > 0, own_sums, scene_is_lean(scene->fast));
     size_t smem = stack_smem_bytes(entries);
-    {
-        const int64_t cells = static_cast<int64_t>(kBands) * p->num_bins * (job.ambisonic_fx ? 4 : 1) + scene->num_surfaces;
-        const int64_t bytes = 4 * (4 * cells + 2 * scene->num_surfaces);
-        if (bytes <= kSharedSumBytes) {
-            table.shared_cells = static_cast<int32_t>(cells);
-            smem += static_cast<size_t>(bytes);
-            // always the same limit, so that concurrent calls do not lower it for one another
-            AC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(stack_smem_bytes(kBvhStack)) + kSharedSumBytes));
-        }
+    table.stack_words = static_cast<int32_t>(smem / sizeof(int));
+    if (own_sums) {
+        table.shared_cells = static_cast<int32_t>(cells);
+        smem += static_cast<size_t>(sum_bytes);
+        // always the same limit, so that concurrent calls do not lower it for one another
+        AC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(stack_smem_bytes(kBvhStack)) + kSharedSumBytes));
     }
     const int grid = fast_grid(kernel, scene->device, block, smem, spread_rays(p->num_rays, table.lanes), p->grid_blocks);
     kernel<<<grid, block, smem, stream>>>(job, scene->fast, table);
     AC_CUDA_TRY(cudaGetLastError());
     const FinalizeTargets tg{o->echogram, job.ambisonic_fx ? o->ambisonic : nullptr, o->surface_energy};
-    const size_t cells = static_cast<size_t>(kBands) * p->num_bins * 5 + scene->num_surfaces;
-    finalize_f32_single_kernel<<<static_cast<int>(std::min<size_t>((cells + 255) / 256, 1024)), 256, 0, stream>>>(job, tg);
+    const size_t results = static_cast<size_t>(kBands) * p->num_bins * 5 + scene->num_surfaces;
+    finalize_f32_single_kernel<<<static_cast<int>(std::min<size_t>((results + 255) / 256, 1024)), 256, 0, stream>>>(job, tg);
     AC_CUDA_TRY(cudaGetLastError());
     return AC_OK;
 }

@@ -802,8 +802,11 @@ __device__ __forceinline__ void winner_normal(const SceneDev<float> &sc, int si,
 // the sum of their high halves, each as two 32-bit words (the same sums that add_fixed forms in the outputs), then the
 // hit and contribution counts of the surfaces.  Cells: the echogram [6, bins], the three directional ambisonic channels
 // [6, 3, bins], the surfaces' energies.  All rays of a small room deposit into a few hundred addresses, and at L2 those
-// atomics queue up behind one another (shoebox, 100 bins, 50 bounces: 100,000 rays 3.57 ms into the outputs, 0.43 here;
-// 400,000 rays 13.3 and 1.28).
+// atomics queue up behind one another (shoebox, 100 bins, 50 bounces: 100,000 rays 2.75 ms into the outputs, 0.39 here;
+// 400,000 rays 9.7 and 1.13; with ambisonics 1,000 / 400,000 rays 0.36 / 14.2 and 0.38 / 1.57).  Where the deposits are
+// spread out, it takes no longer (U room, 100,000 / 400,000 rays 0.80 / 1.80 and 0.72 / 1.77; with ambisonics 0.81 / 2.3
+// and 0.82 / 2.04).  What bounds an addition is the latency of its old values and the instructions: taken one after
+// another, carry by carry, the shoebox took 0.42 / 1.24 ms, and with ambisonics 0.53 / 2.12.
 struct SharedSums {
     unsigned *words;
     int cells;
@@ -813,20 +816,23 @@ struct SharedSums {
         words = reinterpret_cast<unsigned *>(stack_words) + t.stack_words;
     }
 
-    __device__ __forceinline__ void add(int cell, long long q) const {
-        if (q == 0) return;
-        const unsigned lo = static_cast<unsigned>(q), hi = static_cast<unsigned>(q >> 32);
-        unsigned *w = words + cell;
-        if (lo) {
-            const unsigned old = atomicAdd(w, lo);
-            if (old + lo < old) atomicAdd(w + cells, 1u);
+    // Adds q[i] to cell `first` + i * `step`: all sums of the halves first, whose old values then tell the carries.
+    template <int N>
+    __device__ __forceinline__ void add(int first, int step, const long long (&q)[N]) const {
+        unsigned *w = words + first;
+        unsigned low[N], high[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            low[i] = atomicAdd(w + i * step, static_cast<unsigned>(q[i]));
+            high[i] = atomicAdd(w + 2 * cells + i * step, static_cast<unsigned>(q[i] >> 32));
         }
-        unsigned top = q < 0 ? 0xFFFFFFFFu : 0u;   // the high half is signed
-        if (hi) {
-            const unsigned old = atomicAdd(w + 2 * cells, hi);
-            top += old + hi < old ? 1u : 0u;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const unsigned lo = static_cast<unsigned>(q[i]), hi = static_cast<unsigned>(q[i] >> 32);
+            if (low[i] + lo < lo) atomicAdd(w + cells + i * step, 1u);
+            const unsigned top = (q[i] < 0 ? 0xFFFFFFFFu : 0u) + (high[i] + hi < hi ? 1u : 0u);   // the high half is signed
+            if (top) atomicAdd(w + 3 * cells + i * step, top);
         }
-        if (top) atomicAdd(w + 3 * cells, top);
     }
 
     __device__ __forceinline__ unsigned *hits() const { return words + 4 * cells; }
@@ -859,40 +865,55 @@ struct SharedSums {
 };
 
 // Where a lane's deposits go: the block's shared accumulators, or the job's accumulators in global memory (in a batch
-// the block's copy of them, see Job::shard_mask).
-template <bool kSingle, bool kShards>
+// the block's copy of them, see Job::shard_mask).  kOwnSums: the block's own sums, so in a single-job launch those in
+// shared memory.  The two kinds are kernels of their own: with the choice made at each deposit the code of both stood 24
+// times in an ambisonic kernel (U room, 107 bins, 100,000 / 400,000 rays x 50 bounces into the outputs 0.93 / 2.67 ms,
+// now 0.81 / 2.59).
+template <bool kSingle, bool kOwnSums>
 struct Deposit {
     const Job<float> &job;
     const FastTable &table;
     size_t shard;
 
     __device__ __forceinline__ Deposit(const Job<float> &j, const FastTable &t) : job(j), table(t), shard(0) {
-        if (kShards) shard = static_cast<size_t>(blockIdx.x & job.shard_mask) * job.shard_stride;
+        if (!kSingle && kOwnSums) shard = static_cast<size_t>(blockIdx.x & job.shard_mask) * job.shard_stride;
     }
-    __device__ __forceinline__ bool shared() const { return kSingle && table.shared_cells > 0; }
+    static constexpr bool kShared = kSingle && kOwnSums;
 
-    // Echogram cell band * bins + bin.
-    __device__ __forceinline__ void add(int cell, long long q) const {
-        if (shared()) SharedSums(table).add(cell, q);
-        else add_fixed(job.echogram_fx + shard + 2 * static_cast<size_t>(cell), q);
+    // A band's quanta of bin `bin`: the echogram's and, with ambisonics, the three directional channels'.
+    __device__ __forceinline__ void add(int band, int bin, long long q) const {
+        const int cell = band * job.num_bins + bin;
+        if constexpr (kShared) {
+            const long long all[1] = {q};
+            SharedSums(table).add(cell, 0, all);
+        } else {
+            add_fixed(job.echogram_fx + shard + 2 * static_cast<size_t>(cell), q);
+        }
     }
-    // Directional ambisonic channel 1 + axis of a band and bin; `cell`: its shared cell.
-    __device__ __forceinline__ void add_direction(int cell, int band, int axis, int bin, long long q) const {
-        if (shared()) SharedSums(table).add(cell, q);
-        else add_fixed(job.ambisonic_fx + shard + 2 * (static_cast<size_t>(band * 4 + 1 + axis) * job.num_bins + bin), q);
+    __device__ __forceinline__ void add(int band, int bin, long long q, const long long (&direction)[3]) const {
+        add(band, bin, q);
+        if constexpr (kShared) {
+            SharedSums(table).add((kBands + 3 * band) * job.num_bins + bin, job.num_bins, direction);
+        } else {
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                add_fixed(job.ambisonic_fx + shard + 2 * (static_cast<size_t>(band * 4 + 1 + a) * job.num_bins + bin),
+                          direction[a]);
+        }
     }
     __device__ __forceinline__ void add_surface(int surf, long long energy) const {
-        if (shared()) {
+        if constexpr (kShared) {
             const SharedSums sums(table);
             atomicAdd(sums.hits() + job.scene.num_surfaces + surf, 1u);
-            sums.add(sums.cells - job.scene.num_surfaces + surf, energy);
+            const long long all[1] = {energy};
+            sums.add(sums.cells - job.scene.num_surfaces + surf, 0, all);
         } else {
             atomicAdd(job.contrib_counts + shard + surf, 1ull);
             add_fixed(job.surface_energy_fx + shard + 2 * static_cast<size_t>(surf), energy);
         }
     }
     __device__ __forceinline__ void add_hits(int surf, unsigned count) const {
-        if (shared()) atomicAdd(SharedSums(table).hits() + surf, count);
+        if constexpr (kShared) atomicAdd(SharedSums(table).hits() + surf, count);
         else atomicAdd(job.hit_counts + shard + surf, static_cast<unsigned long long>(count));
     }
 };
@@ -957,7 +978,7 @@ __device__ __forceinline__ int find_job_range(const int64_t *prefix, int lo, int
     return lo;
 }
 
-template <bool kSingle, bool kPhilox, bool kAmb, bool kVisual, bool kService = false, bool kShards = false, bool kLean = false>
+template <bool kSingle, bool kPhilox, bool kAmb, bool kVisual, bool kService = false, bool kOwnSums = false, bool kLean = false>
 __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(const __grid_constant__ Job<float> single,
                                                          const __grid_constant__ FastScene single_fast,
                                                          const __grid_constant__ FastTable table) {
@@ -1059,7 +1080,7 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
     bool has = false;
     s.job = 0;
     const bool takes = lane_id < table.lanes;
-    if (kSingle && table.shared_cells > 0) {
+    if constexpr (kSingle && kOwnSums) {
         SharedSums sums(table);
         for (int i = threadIdx.x; i < 4 * table.shared_cells + 2 * single.scene.num_surfaces; i += blockDim.x) sums.words[i] = 0u;
         __syncthreads();
@@ -1317,7 +1338,7 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
                              : __match_any_sync(counting, ((static_cast<unsigned>(s.job) & 1023u) << 22) |
                                                               static_cast<unsigned>(surf));
                 if (lane_id == __ffs(same) - 1)
-                    Deposit<kSingle, kShards>(job, table).add_hits(surf, static_cast<unsigned>(__popc(same)));
+                    Deposit<kSingle, kOwnSums>(job, table).add_hits(surf, static_cast<unsigned>(__popc(same)));
             }
             const float h[3] = {hx, hy, hz};
             make_ray(query, h, sd);
@@ -1355,19 +1376,25 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
                         const float common = job.ray_scale * source_gain * distance_term * (diffuse + specular);
                         long long esum = 0;
                         float energy_sum = 0.0f;
-                        const Deposit<kSingle, kShards> deposit(job, table);
-#pragma unroll
+                        const Deposit<kSingle, kOwnSums> deposit(job, table);
+                        // an ambisonic launch with sums in shared memory goes through the bands one by one (their
+                        // reflectances read again): unrolled, its 24 additions cost instruction fetches (U room, 400,000
+                        // rays 2.66 ms, now 2.04)
+                        constexpr int kUnroll = kAmb && kSingle && kOwnSums ? 1 : kBands;
+#pragma unroll kUnroll
                         for (int b = 0; b < kBands; ++b) {
-                            const float e = common * refl[b] * lane_acc[b * kStackStride];
+                            const float rb = kUnroll == 1 ? __ldg(job.scene.mats + static_cast<size_t>(surf) * kMatStride + b)
+                                                          : refl[b];
+                            const float e = common * rb * lane_acc[b * kStackStride];
                             if (kVisual) energy_sum += e;
                             const long long qe = quantize(e, job.energy_scale);
-                            deposit.add(b * job.num_bins + bin, qe);
-                            if (kAmb) {   // the W channel is the echogram's own sums: the launch's last kernel copies them
-                                const float *d0 = s.d0;
-                                const int a = kBands * job.num_bins + b * 3 * job.num_bins + bin;
-                                deposit.add_direction(a, b, 0, bin, quantize(e * d0[0], job.energy_scale));
-                                deposit.add_direction(a + job.num_bins, b, 1, bin, quantize(e * d0[1], job.energy_scale));
-                                deposit.add_direction(a + 2 * job.num_bins, b, 2, bin, quantize(e * d0[2], job.energy_scale));
+                            if constexpr (kAmb) {   // the W channel is the echogram's own sums: the launch's last kernel copies them
+                                const long long direction[3] = {quantize(e * s.d0[0], job.energy_scale),
+                                                                quantize(e * s.d0[1], job.energy_scale),
+                                                                quantize(e * s.d0[2], job.energy_scale)};
+                                deposit.add(b, bin, qe, direction);
+                            } else {
+                                deposit.add(b, bin, qe);
                             }
                             esum += qe;
                         }
@@ -1463,7 +1490,7 @@ __global__ void __launch_bounds__(256, AC_FAST_MIN_BLOCKS) trace_fast_kernel(con
         const unsigned long long cn = count_n;
         if (cn && service_count(table, cs, cn, lane_id)) service_finish(table, cs, lane_id);
     }
-    if (kSingle && table.shared_cells > 0) {
+    if constexpr (kSingle && kOwnSums) {
         __syncthreads();   // every warp of the block has made its last deposit
         SharedSums(table).flush(single);
     }

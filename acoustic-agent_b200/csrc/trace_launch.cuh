@@ -31,7 +31,9 @@ inline int warp_lanes(int device, int64_t rays, int least) {
 // Rays a launch of full warps would need as many warps for.
 inline int64_t spread_rays(int64_t rays, int lanes) { return (rays + lanes - 1) / lanes * 32; }
 
-constexpr int kSharedSumBytes = 40 * 1024;   // a block's own accumulators at most: three blocks per SM keep an L1 for the scene
+// A block's own accumulators at most: with the lanes' state (10 KB) and stacks of up to 24 entries (24 KB) three blocks
+// per SM keep some L1 for the scene.
+constexpr int kSharedSumBytes = 40 * 1024;
 
 // Reference initial values of the visual-candidate arrays (steam_rt.py:4718-4723).
 template <typename T>
