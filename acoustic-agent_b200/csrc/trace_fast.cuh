@@ -924,7 +924,7 @@ static __device__ __noinline__ int2 fallback_walk(const SceneDev<float> sc, floa
                                                   float dy, float dz) {
     const float o[3] = {ox, oy, oz}, d[3] = {dx, dy, dz};
     float n[3], t;
-    const int surf = closest_hit(sc, true, o, d, t, n);
+    const int surf = closest_hit<float, true, false>(sc, o, d, t, n);
     return make_int2(surf, __float_as_int(t));
 }
 

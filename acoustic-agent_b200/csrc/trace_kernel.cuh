@@ -334,10 +334,10 @@ __device__ __forceinline__ int rec_tag(const T *rec) { return tag_bits(__ldg(rec
 //     4.7 of 9.2 cycles per instruction for instructions (now 2.2).  A linear scene keeps the inlined loops: with few
 //     surfaces they are short, and out of line a shoebox took 10 % longer at 5,000 rays.
 //
-// What bounds it now is divergence: 3 of 32 lanes are active per instruction.  Measured with the rays of a small launch
-// spread over more warps (warp_lanes): furnished U room in BVH mode, 100 bounces, 500 / 5,000 / 20,000 / 100,000 rays
-// 6.36 / 6.25 / 7.01 / 17.1 -> 2.07 / 3.5 / 5.5 / 11.1 ms; apartment, 2,000 / 20,000 rays 11.6 / 12.7 -> 4.1 / 8.3;
-// shoebox, linear, 50 bounces, 500 / 5,000 / 20,000 rays 0.69 / 0.71 / 1.01 -> 0.44 / 0.68 / 1.03.
+// What bounds it now is divergence: 3 of 32 lanes are active per instruction.  Where it pays, and how many lanes take rays,
+// is query_plan's rule; with that, furnished U room in BVH mode, 100 bounces, 500 / 5,000 / 20,000 / 100,000 rays 6.45 /
+// 6.31 / 7.07 / 17.1 -> 1.98 / 3.4 / 5.2 / 10.7 ms; apartment, 2,000 / 20,000 rays 11.6 / 12.7 -> 3.9 / 8.2; shoebox,
+// linear, 50 bounces, 500 / 5,000 / 20,000 rays 0.70 / 0.71 / 1.01 -> 0.43 / 0.63 / 1.01.
 
 __device__ __forceinline__ double approx_inverse(double x) {   // |x| between 1e-30 and 1e30
     return static_cast<double>(__frcp_rn(static_cast<float>(x)));
@@ -459,7 +459,18 @@ __device__ __forceinline__ void normal64(const SceneDev<double> &sc, int surface
         n[2] = __ldg(sc.normals + 3 * surface + 2);
     } else {
         const double *rec = sc.prims_linear + static_cast<size_t>(surface) * kPrimStride;
-        exact_hit(rec, rec_tag(rec) & 3, o, d, sc.corners, sc.num_corners, n);
+        const int kind = rec_tag(rec) & 3;
+        if (kind == 2) {
+            const double at[3] = {o[0], o[1], o[2]}, along[3] = {d[0], d[1], d[2]};   // copies: the lane's own stay in registers
+            double normal[3];
+            exact_hit(rec, kind, at, along, sc.corners, sc.num_corners, normal);
+            n[0] = normal[0]; n[1] = normal[1]; n[2] = normal[2];
+        } else {   // a wall's or a polygon's normal is its own, wherever it is hit
+            const int at = kind == 0 ? 6 : 1;
+            n[0] = __ldg(rec + at);
+            n[1] = __ldg(rec + at + 1);
+            n[2] = __ldg(rec + at + 2);
+        }
     }
     const double dot = n[0] * d[0] + n[1] * d[1] + n[2] * d[2];
     if (dot > 0.0) { n[0] = -n[0]; n[1] = -n[1]; n[2] = -n[2]; }
@@ -468,14 +479,13 @@ __device__ __forceinline__ void normal64(const SceneDev<double> &sc, int surface
 // Closest hit: steam_rt.py:4429-4478 (linear) and :4481-4506 (escape-link walk).
 // The BVH walk keeps the reference's tie rule, including its side effect that a
 // ray missing every visited surface returns the lowest visited index with t=1e30.
-template <typename T>
-__device__ __forceinline__ int closest_hit(const SceneDev<T> &sc, bool use_bvh, const T *o, const T *d, T &t_out,
-                                           T *n_out) {
+template <typename T, bool kTree, bool kSift>
+__device__ __forceinline__ int closest_hit(const SceneDev<T> &sc, const T *o, const T *d, T &t_out, T *n_out) {
     T best_t = T(1e30);
     int best = -1;
     T bn[3] = {T(0), T(0), T(0)};
     T n[3];
-    if (use_bvh) {
+    if constexpr (kTree) {
         int node = 0;
         while (node < sc.num_nodes) {
             const T *np = sc.nodes + static_cast<size_t>(node) * kNodeStride;
@@ -506,10 +516,11 @@ __device__ __forceinline__ int closest_hit(const SceneDev<T> &sc, bool use_bvh, 
             bn[2] = __ldg(sc.normals + 3 * best + 2);
         }
     } else {
-        const double inv_z = approx_inverse(static_cast<double>(fabs(d[2]) < T(1e-30) ? T(1e-30) : d[2]));
+        double inv_z = 0.0;
+        if constexpr (kSift) inv_z = approx_inverse(fabs(d[2]) < 1e-30 ? 1e-30 : d[2]);
         for (int si = 0; si < sc.num_surfaces; ++si) {
             const T *rec = sc.prims_linear + static_cast<size_t>(si) * kPrimStride;
-            if constexpr (sizeof(T) == 8) {
+            if constexpr (kSift) {
                 if (!maybe_hit(rec, rec_tag(rec) & 3, o, d, inv_z, best_t)) continue;
             }
             const T t = surface_hit(rec, rec_tag(rec) & 3, o, d, sc.corners, sc.num_corners, n);
@@ -527,10 +538,10 @@ __device__ __forceinline__ int closest_hit(const SceneDev<T> &sc, bool use_bvh, 
 
 // Shadow query: is any surface hit strictly closer than max_t?  Equivalent to the
 // reference's `closest t < distance - EPS` test (steam_rt.py:4794).
-template <typename T>
-__device__ __forceinline__ bool any_hit(const SceneDev<T> &sc, bool use_bvh, const T *o, const T *d, T max_t) {
+template <typename T, bool kTree, bool kSift>
+__device__ __forceinline__ bool any_hit(const SceneDev<T> &sc, const T *o, const T *d, T max_t) {
     T n[3];
-    if (use_bvh) {
+    if constexpr (kTree) {
         int node = 0;
         while (node < sc.num_nodes) {
             const T *np = sc.nodes + static_cast<size_t>(node) * kNodeStride;
@@ -553,10 +564,11 @@ __device__ __forceinline__ bool any_hit(const SceneDev<T> &sc, bool use_bvh, con
         }
         return false;
     }
-    const double inv_z = approx_inverse(static_cast<double>(fabs(d[2]) < T(1e-30) ? T(1e-30) : d[2]));
+    double inv_z = 0.0;
+    if constexpr (kSift) inv_z = approx_inverse(fabs(d[2]) < 1e-30 ? 1e-30 : d[2]);
     for (int si = 0; si < sc.num_surfaces; ++si) {
         const T *rec = sc.prims_linear + static_cast<size_t>(si) * kPrimStride;
-        if constexpr (sizeof(T) == 8) {
+        if constexpr (kSift) {
             if (!maybe_hit(rec, rec_tag(rec) & 3, o, d, inv_z, max_t)) continue;
         }
         const T t = surface_hit(rec, rec_tag(rec) & 3, o, d, sc.corners, sc.num_corners, n);
@@ -686,6 +698,11 @@ __device__ __forceinline__ void warp_count(unsigned mask, unsigned long long key
     if ((threadIdx.x & 31) == leader) atomicAdd(target, static_cast<unsigned long long>(total));
 }
 
+// How a launch of trace_kernel answers its queries; the results are the same.  kLoop, kTree: the reference's loop and its
+// walk of the tree, kBoth: as each job asks.  kSifted, kWalk: with the approximate tests before the exact ones, kMixed: as
+// each job asks.
+enum class Query { kLoop, kTree, kBoth, kSifted, kWalk, kMixed };
+
 template <typename T>
 struct Lane {
     T o[3];
@@ -701,7 +718,7 @@ struct Lane {
     int vslot;   // visual-candidate slot, -1 for none
 };
 
-template <typename T, bool kSingle>
+template <typename T, bool kSingle, Query kQuery>
 __global__ void __launch_bounds__(256) trace_kernel(const __grid_constant__ Job<T> single,
                                                     const __grid_constant__ BatchTable table) {
     const unsigned full = 0xFFFFFFFFu;
@@ -768,15 +785,17 @@ __global__ void __launch_bounds__(256) trace_kernel(const __grid_constant__ Job<
         if (has) {
             const Job<T> &job = kSingle ? single : jobs[s.job];
             const SceneDev<T> &sc = job.scene;
-            const bool bvh = job.use_bvh != 0;
+            constexpr bool kSift = kQuery == Query::kSifted || kQuery == Query::kMixed;
+            const bool walk = kQuery == Query::kWalk || (kQuery == Query::kMixed && job.use_bvh != 0);
+            const bool tree = kQuery == Query::kTree || (kQuery == Query::kBoth && job.use_bvh != 0);
             T t, n[3] = {T(0), T(0), T(0)};
             int surf;
-            if (bvh) {
+            if (walk) {
                 const Walk64 hit = walk64(sc, false, s.o[0], s.o[1], s.o[2], s.d[0], s.d[1], s.d[2], 1e30);
                 surf = hit.surface;
                 t = hit.t;
             } else {
-                surf = closest_hit(sc, false, s.o, s.d, t, n);
+                surf = tree ? closest_hit<T, true, kSift>(sc, s.o, s.d, t, n) : closest_hit<T, false, kSift>(sc, s.o, s.d, t, n);
             }
             s.queries += 1;
             bool dead = surf < 0 || t <= job.listener_radius || s.path > job.max_path_length;
@@ -790,7 +809,7 @@ __global__ void __launch_bounds__(256) trace_kernel(const __grid_constant__ Job<
                 finished = true;
             } else {
                 count_surface = surf;
-                if (bvh) normal64(sc, surf, t, s.o, s.d, n);
+                if (walk) normal64(sc, surf, t, s.o, s.d, n);
                 if (job.ray_surfaces)
                     job.ray_surfaces[s.ray * job.num_bounces + s.bounce] = surf;
                 const T hx = s.o[0] + t * s.d[0] + T(1e-2) * n[0];
@@ -810,10 +829,11 @@ __global__ void __launch_bounds__(256) trace_kernel(const __grid_constant__ Job<
                         const T h[3] = {hx, hy, hz};
                         s.shadows += 1;
                         bool occluded;
-                        if (bvh)
+                        if (walk)
                             occluded = walk64(sc, true, h[0], h[1], h[2], sd[0], sd[1], sd[2], dist - 1e-6).surface >= 0;
                         else
-                            occluded = any_hit(sc, false, h, sd, dist - T(1e-6));
+                            occluded = tree ? any_hit<T, true, kSift>(sc, h, sd, dist - T(1e-6))
+                                            : any_hit<T, false, kSift>(sc, h, sd, dist - T(1e-6));
                         if (!occluded) {
                             const T diffuse = T(1.0 / kPi) * scat * facing;
                             T half[3];

@@ -17,14 +17,13 @@ namespace ac {
 constexpr int kDefaultBlock = 256;
 
 // Lanes of a warp that take rays.  A launch too small to fill the GPU is bound by the time of one warp's bounces, which
-// falls with the lanes it carries (its queries end with the slowest lane's), so its rays are spread over up to two
-// warps per scheduler (furnished U room, 100 bounces: 2,000 rays 0.98 -> 0.77 ms, 10,000 rays 1.06 -> 0.88; with three
-// warps 0.92, and 30,000 rays get slower).  Fewer lanes than `least` gain nothing: 4 where the rays of a warp descend a
-// BVH on their own, 16 in the lockstep scan (shoebox, 10,000 rays 0.36 -> 0.33 ms; 0.35 with 8).  The float64 walks are
-// so much longer than what their lanes share that a warp per ray pays: with at least 1 / 2 / 4 / 8 / 32 lanes, U room,
-// 500 rays 2.07 / 2.40 / 2.83 / 3.30 / 5.08 ms, shoebox, 500 rays 0.44 / 0.49 / 0.53 / 0.58 / 0.67.
-inline int warp_lanes(int device, int64_t rays, int least) {
-    const int64_t warps = static_cast<int64_t>(device_sm_count(device)) * 8;
+// falls with the lanes it carries (its queries end with the slowest lane's), so its rays are spread over up to `per_sm`
+// warps per SM.  In float32 two per scheduler (furnished U room, 100 bounces: 2,000 rays 0.98 -> 0.77 ms, 10,000 rays
+// 1.06 -> 0.88; with three warps 0.92, and 30,000 rays get slower), and fewer lanes than `least` gain nothing: 4 where the
+// rays of a warp descend a BVH on their own, 16 in the lockstep scan (shoebox, 10,000 rays 0.36 -> 0.33 ms; 0.35 with 8).
+// In float64: query_plan.
+inline int warp_lanes(int device, int64_t rays, int least, int per_sm = 8) {
+    const int64_t warps = static_cast<int64_t>(device_sm_count(device)) * per_sm;
     return static_cast<int>(std::min<int64_t>(32, std::max<int64_t>(least, (rays + warps - 1) / warps)));
 }
 
@@ -177,16 +176,64 @@ inline void fill_job(const ac_scene_s *scene, const ac_trace_params *p, const ac
     }
 }
 
-template <typename T, bool kSingle>
-inline int persistent_grid(int device, int block, int64_t total_rays, int requested) {
+template <typename Kernel>
+inline int persistent_grid(Kernel kernel, int device, int block, int64_t total_rays, int requested) {
     int per_sm = 0;
-    cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<T, kSingle>, block, 0);
+    cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0);
     if (err != cudaSuccess || per_sm < 1) per_sm = 1;
     int grid = per_sm * device_sm_count(device);
     if (requested > 0) grid = requested;
     const int64_t needed = (total_rays + block - 1) / block;
     if (needed < grid) grid = static_cast<int>(needed > 0 ? needed : 1);
     return grid;
+}
+
+// How a float64 launch answers its queries and how many lanes of a warp take rays.
+struct QueryPlan {
+    Query query;
+    int lanes;
+};
+
+// `surfaces`: of the launch's largest scene; `loops`, `trees`: whether some of its jobs ask for the linear loop, for the
+// tree; `spread` false: full warps, for a grid that the caller chose.
+//
+// What the approximate tests save is what every lane of a warp skips, so they pay with few lanes or many surfaces, and cost
+// otherwise: with 100,000 rays in a room of 18 surfaces the loop takes 3.4 ms without them and 4.9 with them, in a U room
+// of 30 4.9 and 5.3, in an apartment of 104 8.6 and 7.6; the tree of a room of 9 4.4 and 6.1, of 12 5.8 and 6.7, of 18 9.7
+// and 7.9.  Fewer than 32 lanes pay for as long as queries end at very different times: the U room's tree, 9,600 rays, 2.44
+// ms over eight warps per SM, 2.73 over four, 3.14 over two; but rooms of 22, 9 and 6 surfaces 2.99, 2.58, 2.89; 2.11,
+// 1.70, 1.54 and 1.18, 1.02, 0.97.  The kernels that call the walk hold 194 registers and more, one block per SM: a loop
+// of up to some 47,000 rays is as fast in kMixed, or faster (46 surfaces, 28,800 rays 3.18 ms against 3.24 in kSifted),
+// above it needs two blocks (104 surfaces, 100,000 rays 9.7 and 7.6).  kBoth is a batch's exact loop: kLoop, compiled
+// for batches, takes 3 % longer.
+inline QueryPlan query_plan(int device, int64_t rays, int64_t surfaces, bool loops, bool trees, bool single, bool spread) {
+    const auto lanes = [&](int per_sm) { return spread ? warp_lanes(device, rays, 1, per_sm) : 32; };
+    const int64_t per_warp = rays / (static_cast<int64_t>(device_sm_count(device)) * 8);   // rays per warp, of eight per SM
+    const int few = lanes(8);
+    if (loops && trees) {
+        if (surfaces > 24 || per_warp < 4) return {Query::kMixed, few};
+        return {Query::kBoth, lanes(2)};
+    }
+    if (trees) {
+        if (surfaces > 24 || per_warp < 2) return {Query::kWalk, few};
+        if (surfaces > 12) return {Query::kWalk, per_warp < 4 ? few : lanes(4)};
+        return {per_warp < 9 ? Query::kWalk : Query::kTree, lanes(2)};
+    }
+    const Query exact = single ? Query::kLoop : Query::kBoth;
+    if (surfaces > 64) return {per_warp < 40 ? Query::kMixed : Query::kSifted, few};
+    if (surfaces > 24) return {per_warp < 40 ? Query::kMixed : exact, per_warp < 4 ? few : lanes(4)};
+    return {per_warp < 9 ? Query::kMixed : exact, per_warp < 2 ? few : lanes(2)};
+}
+
+template <typename T, bool kSingle>
+inline auto query_kernel(Query query) {
+    switch (query) {
+        case Query::kTree: return &trace_kernel<T, kSingle, Query::kTree>;
+        case Query::kSifted: return &trace_kernel<T, kSingle, Query::kSifted>;
+        case Query::kWalk: return &trace_kernel<T, kSingle, Query::kWalk>;
+        case Query::kMixed: return &trace_kernel<T, kSingle, Query::kMixed>;
+        default: return &trace_kernel<T, kSingle, kSingle ? Query::kLoop : Query::kBoth>;
+    }
 }
 
 // Single job: the job travels in the kernel's parameter space, so the call
@@ -216,9 +263,12 @@ inline int launch_single(const ac_scene_s *scene, const ac_trace_params *p, cons
     if (block % 32 != 0 || block > 256) return fail(AC_ERR_INVALID, "block_size must be a multiple of 32 up to 256");
     if (p->num_rays > 0) {
         BatchTable none{};
-        none.lanes = p->grid_blocks > 0 ? 32 : warp_lanes(scene->device, p->num_rays, 1);
-        const int grid = persistent_grid<T, true>(scene->device, block, spread_rays(p->num_rays, none.lanes), p->grid_blocks);
-        trace_kernel<T, true><<<grid, block, 0, stream>>>(job, none);
+        const QueryPlan plan = query_plan(scene->device, p->num_rays, scene->num_surfaces, !p->use_bvh, p->use_bvh != 0,
+                                          true, p->grid_blocks <= 0);
+        const auto kernel = query_kernel<T, true>(plan.query);
+        none.lanes = plan.lanes;
+        const int grid = persistent_grid(kernel, scene->device, block, spread_rays(p->num_rays, none.lanes), p->grid_blocks);
+        kernel<<<grid, block, 0, stream>>>(job, none);
         AC_CUDA_TRY(cudaGetLastError());
     }
     return AC_OK;
@@ -306,9 +356,12 @@ inline int launch_batch(const ac_job *jobs_in, const int32_t *indices, int32_t c
     Job<T> *jobs = reinterpret_cast<Job<T> *>(host + off_jobs);
     FinalizeTargets *targets = reinterpret_cast<FinalizeTargets *>(host + off_targets);
     int device = -1;
-    int64_t total = 0;
+    bool loops = false, trees = false;
+    int64_t total = 0, surfaces = 0;
     for (int32_t k = 0; k < count; ++k) {
         const ac_job &in = jobs_in[indices[k]];
+        (in.params.use_bvh ? trees : loops) = true;
+        surfaces = std::max<int64_t>(surfaces, in.scene->num_surfaces);
         if (device < 0) device = in.scene->device;
         if (in.scene->device != device) return fail(AC_ERR_INVALID, "batch jobs must share one device");
         double scale = in.params.energy_scale;
@@ -342,11 +395,13 @@ inline int launch_batch(const ac_job *jobs_in, const int32_t *indices, int32_t c
         table.num_jobs = count;
         table.total_rays = total;
         table.work_counter = counter;
-        table.lanes = cfg && cfg->grid_blocks > 0 ? 32 : warp_lanes(device, total, 1);
-        const int grid = persistent_grid<T, false>(device, block, spread_rays(total, table.lanes), cfg ? cfg->grid_blocks : 0);
+        const QueryPlan plan = query_plan(device, total, surfaces, loops, trees, false, !(cfg && cfg->grid_blocks > 0));
+        const auto kernel = query_kernel<T, false>(plan.query);
+        table.lanes = plan.lanes;
+        const int grid = persistent_grid(kernel, device, block, spread_rays(total, table.lanes), cfg ? cfg->grid_blocks : 0);
         Job<T> unused;
         std::memset(&unused, 0, sizeof(unused));
-        trace_kernel<T, false><<<grid, block, 0, stream>>>(unused, table);
+        kernel<<<grid, block, 0, stream>>>(unused, table);
         AC_CUDA_TRY(cudaGetLastError());
     }
     {
