@@ -35,7 +35,8 @@ struct Offsets {
 };
 
 // Unless the caller chooses, a single room (at most kAutoHybridWalls walls) with any box traces in hybrid mode, its walls
-// in lockstep and its boxes in a BVH; other scenes of more than kAutoBvhSurfaces walls and boxes in BVH mode.  Measured on
+// in lockstep and its boxes in a BVH; other scenes of more than kAutoBvhSurfaces walls and boxes in BVH mode.  A room of no
+// more than kAutoBvhSurfaces never needs a stack: a launch with a shallower one than its tree needs scans it.  Measured on
 // B200: a 4-wall room, 10,000 / 400,000 rays: with 1 box scan 0.466 / 2.24 ms, hybrid 0.456 / 2.19, with 12 boxes scan
 // 0.668 / 2.60, hybrid 0.554 / 2.27, BVH 0.548 / 2.46; U room (8 walls, 20 boxes) hybrid 11.4 ms < BVH 11.8 < scan 12.3;
 // 8-room apartment (52 walls, 374 boxes) BVH 5.1 ms < hybrid 6.3 < scan 9.6 (the last two by earlier kernels).
@@ -322,6 +323,7 @@ int pack_and_upload(const ac_scene_desc *d, const ac_bvh &bvh, const FastLists *
         s->fast.num_polys = static_cast<int32_t>(f->polys.size());
         s->fast.num_box_clusters = static_cast<int32_t>(f->box_clusters.size());
         s->num_clusters = static_cast<int64_t>(f->wall_clusters.size() + f->box_clusters.size());
+        s->scan = s->fast;
         if (f->use_bvh) {
             // BVH mode: walls and boxes come from the traversal BVH, only polygons stay in the scan;
             // hybrid mode: boxes from the BVH, walls and polygons in the scan
@@ -489,6 +491,8 @@ extern "C" int ac_scene_create(const ac_scene_desc *d, ac_scene_t *out) {
     s->bvh_nodes = lists.use_bvh ? lists.bvh.num_nodes() : 0;
     s->bvh_width = lists.use_bvh ? lists.bvh.width : 0;
     s->bvh_stack_need = lists.use_bvh ? lists.bvh.stack_need : 0;
+    s->scan_too = d->traversal == AC_TRAVERSAL_AUTO && lists.hybrid &&
+                  static_cast<int64_t>(lists.wall_slots.size() + lists.box_slots.size()) <= kAutoBvhSurfaces;
     rc = pack_and_upload<float>(d, bvh, &lists, blo, bhi, s, &s->storage_f32, &s->bytes_f32, &s->f32);
     if (rc == AC_OK)
         rc = pack_and_upload<double>(d, bvh, nullptr, blo, bhi, s, &s->storage_f64, &s->bytes_f64, &s->f64);

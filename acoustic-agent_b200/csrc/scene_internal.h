@@ -34,6 +34,10 @@ struct ac_scene_s {
     int64_t bvh_nodes = 0;
     int32_t bvh_width = 0;
     int32_t bvh_stack_need = 0;
+    // A room that AUTO would scan whole but for its boxes' tree (kAutoBvhSurfaces): its scan form, which launches with a
+    // shallower stack than the tree needs trace.
+    bool scan_too = false;
+    ac::FastScene scan{};
     double max_reflection = 0.0;   // bound used when choosing the fixed-point scale
     double max_scattering = 0.0;
     double min_scattering = 0.0;
@@ -53,6 +57,13 @@ template <>
 inline const SceneDev<float> &scene_view<float>(const ac_scene_s *s) { return s->f32; }
 template <>
 inline const SceneDev<double> &scene_view<double>(const ac_scene_s *s) { return s->f64; }
+
+// The form of a scene that a float32 launch traces, `entries` stack entries asked for (0: the library's choice), and the
+// stack that this form needs (0: none).
+inline const FastScene &fast_form(const ac_scene_s *s, int entries) {
+    return s->scan_too && entries > 0 && entries < s->bvh_stack_need ? s->scan : s->fast;
+}
+inline int stack_need(const ac_scene_s *s, const FastScene &form) { return form.num_bvh_nodes > 0 ? s->bvh_stack_need : 0; }
 
 // Power-of-two fixed-point scale: the largest deposit the scene and parameters
 // allow, summed over the six bands, maps to at most 2^62.

@@ -260,7 +260,7 @@ extern "C" int ac_service_submit(ac_service_t s, const ac_job *jobs, int32_t num
             return ac::fail(AC_ERR_INVALID, "job %d: the service traces float32 Philox jobs without ambisonics, "
                             "visual candidates or recorded rays", j);
         if (in.params.num_bounces < 1) return ac::fail(AC_ERR_INVALID, "job %d: needs at least one bounce", j);
-        if (in.scene->fast.num_bvh_nodes > 0 && in.scene->bvh_stack_need > s->stack_entries)
+        if (ac::stack_need(in.scene, ac::fast_form(in.scene, s->stack_entries)) > s->stack_entries)
             return ac::fail(AC_ERR_INVALID, "job %d: its scene needs %d traversal stack entries, the service has %d",
                             j, in.scene->bvh_stack_need, s->stack_entries);
     }
@@ -286,7 +286,7 @@ extern "C" int ac_service_submit(ac_service_t s, const ac_job *jobs, int32_t num
         if (!(scale > 0.0)) scale = ac::choose_energy_scale(in.scene, &in.params);
         if (in.outputs.scale_out) *in.outputs.scale_out = scale;
         ac::fill_job<float>(in.scene, &in.params, &in.outputs, scale, sl.job);
-        sl.fast = in.scene->fast;
+        sl.fast = ac::fast_form(in.scene, s->stack_entries);
         sl.echogram = in.outputs.echogram;
         sl.surface_energy = in.outputs.surface_energy;
         sl.seq = seq;

@@ -242,8 +242,8 @@ int launch_trace_f32(const ac_scene_s *scene, const ac_trace_params *p, const ac
                      void *stream_ptr) {
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
     int entries = 0;
-    const int rc = launch_stack_entries(p->stack_entries, scene->fast.num_bvh_nodes > 0 ? scene->bvh_stack_need : 0,
-                                        &entries);
+    const FastScene &form = fast_form(scene, p->stack_entries);
+    const int rc = launch_stack_entries(p->stack_entries, stack_need(scene, form), &entries);
     if (rc != AC_OK) return rc;
     Job<float> job;
     fill_job<float>(scene, p, o, scale, job);
@@ -256,7 +256,7 @@ int launch_trace_f32(const ac_scene_s *scene, const ac_trace_params *p, const ac
     const int block = p->block_size > 0 ? p->block_size : kDefaultBlock;
     if (block % 32 != 0 || block > 256) return fail(AC_ERR_INVALID, "block_size must be a multiple of 32 up to 256");
     FastTable table{};
-    table.lanes = p->grid_blocks > 0 ? 32 : warp_lanes(scene->device, p->num_rays, scene->fast.num_bvh_nodes > 0 ? 4 : 16);
+    table.lanes = p->grid_blocks > 0 ? 32 : warp_lanes(scene->device, p->num_rays, form.num_bvh_nodes > 0 ? 4 : 16);
     table.chunk_rays = std::min(kDefaultChunkRays, table.lanes);
     table.chunk_counter = reinterpret_cast<unsigned long long *>(o->counters) + 4;
     const int64_t cells = static_cast<int64_t>(kBands) * p->num_bins * (job.ambisonic_fx ? 4 : 1) + scene->num_surfaces;
@@ -264,9 +264,9 @@ int launch_trace_f32(const ac_scene_s *scene, const ac_trace_params *p, const ac
     const bool own_sums = sum_bytes <= kSharedSumBytes;
     // beside the sums no deeper stack than the tree uses, so that three blocks still fit an SM (U room, 400 bins, 100,000
     // rays: 0.98 ms with two, 0.72 with three; what lies above the need is never read)
-    if (own_sums) entries = std::min(entries, static_cast<int>(scene->bvh_stack_need));
+    if (own_sums) entries = std::min(entries, stack_need(scene, form));
     const FastKernel kernel = pick_kernel<true>(p->rng_mode == AC_RNG_PHILOX, p->render_ambisonics != 0,
-                                                p->visual_limit > 0, own_sums, scene_is_lean(scene->fast));
+                                                p->visual_limit > 0, own_sums, scene_is_lean(form));
     size_t smem = stack_smem_bytes(entries);
     table.stack_words = static_cast<int32_t>(smem / sizeof(int));
     if (own_sums) {
@@ -277,7 +277,7 @@ int launch_trace_f32(const ac_scene_s *scene, const ac_trace_params *p, const ac
                                          static_cast<int>(stack_smem_bytes(kBvhStack)) + kSharedSumBytes));
     }
     const int grid = fast_grid(kernel, scene->device, block, smem, spread_rays(p->num_rays, table.lanes), p->grid_blocks);
-    kernel<<<grid, block, smem, stream>>>(job, scene->fast, table);
+    kernel<<<grid, block, smem, stream>>>(job, form, table);
     AC_CUDA_TRY(cudaGetLastError());
     const FinalizeTargets tg{o->echogram, job.ambisonic_fx ? o->ambisonic : nullptr, o->surface_energy};
     const size_t results = static_cast<size_t>(kBands) * p->num_bins * 5 + scene->num_surfaces;
@@ -324,13 +324,14 @@ int launch_batch_f32(const ac_job *jobs_in, const int32_t *indices, int32_t coun
         const ac_job &in = jobs_in[order[k]];
         if (device < 0) device = in.scene->device;
         if (in.scene->device != device) return fail(AC_ERR_INVALID, "batch jobs must share one device");
-        if (in.scene->fast.num_bvh_nodes > 0) need = std::max(need, in.scene->bvh_stack_need);
-        lean = lean && scene_is_lean(in.scene->fast);
+        const FastScene &form = fast_form(in.scene, cfg ? cfg->stack_entries : 0);
+        need = std::max(need, stack_need(in.scene, form));
+        lean = lean && scene_is_lean(form);
         if (in.scene != current || groups[g].num_jobs >= kMaxGroupJobs) {
             ++g;
             current = in.scene;
             group_rays[g] = total;
-            groups[g] = FastGroup{in.scene->f32, in.scene->fast, k, 0};
+            groups[g] = FastGroup{in.scene->f32, form, k, 0};
         }
         groups[g].num_jobs += 1;
         double scale = in.params.energy_scale;

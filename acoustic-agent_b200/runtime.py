@@ -54,6 +54,7 @@ def _stream_ptr(stream: torch.cuda.Stream | None) -> ctypes.c_void_p:
 
 
 MAX_STACK_ENTRIES = 32   # traversal stack entries per lane at most (the library's kBvhStack)
+SCAN_SURFACES = 16       # AUTO rooms of no more walls and boxes need no stack (the library's kAutoBvhSurfaces)
 
 
 class DeviceScene:
@@ -122,6 +123,11 @@ class DeviceScene:
         # traversal stack entries per lane that launches over this scene use unless told otherwise (a tuned
         # schedule knob; 0: the library's maximum)
         self.stack_entries = int(stack_entries) if self.bvh_nodes > 0 else 0
+        # a small room that AUTO gave a tree is scanned where the stack is too shallow for it: it asks for no depth
+        self.stack_optional = (traversal == "auto" and self.traversal == "hybrid" and
+                               int(np.count_nonzero(keep["kinds"] != 1)) <= SCAN_SURFACES)
+        if self.stack_optional and not self.bvh_stack_need <= self.stack_entries <= MAX_STACK_ENTRIES:
+            self.stack_entries = 0
         self.max_reflection = float(np.max(keep["reflection"])) if S else 0.0
         # events recorded after CUDA-graph replays that read this scene (the library tracks eager launches
         # itself, not work captured into a graph); close() waits for them
@@ -449,8 +455,9 @@ class BatchWorkspace(_StagedWorkspace):
 
 def launch_stack_entries(scenes: Sequence[DeviceScene]) -> int:
     """Stack entries of one launch over `scenes`: the largest of the BVH scenes' choices, or 0 (the library's
-    maximum) when one of them has none."""
-    prefs = [s.stack_entries for s in scenes if s.bvh_nodes > 0]
+    maximum) when one of them has none.  Rooms that need no stack (stack_optional) count with their choice only."""
+    prefs = [s.stack_entries for s in scenes
+             if s.bvh_nodes > 0 and (s.stack_entries or not getattr(s, "stack_optional", False))]
     return max(prefs) if prefs and all(prefs) else 0
 
 

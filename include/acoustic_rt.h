@@ -127,7 +127,8 @@ typedef struct ac_scene_info {
     int64_t bvh_nodes;           /* float32 BVH: inner nodes (0 in scan mode) */
     int32_t bvh_width;           /* float32 BVH: children per inner node (0 in scan mode) */
     int32_t bvh_stack_need;      /* float32 BVH: traversal stack entries a ray can need, the sentinel
-                                    included (the least `stack_entries` a launch over it may use) */
+                                    included (the least `stack_entries` a launch over it may use, but
+                                    see ac_trace_params::stack_entries) */
 } ac_scene_info;
 
 /* One trace: rays from the listener, next-event estimation to the source.
@@ -175,6 +176,8 @@ typedef struct ac_trace_params {
     /* Float32 BVH scenes: entries of each lane's traversal stack (shared
      * memory, 1 KiB per entry per 256-thread block).  0: the library maximum
      * (32); otherwise bvh_stack_need of the scene .. 32, else AC_ERR_INVALID.
+     * A room of at most 16 walls and boxes whose traversal AUTO chose takes any
+     * 1 .. 32: below its bvh_stack_need it is scanned.
      * A schedule knob: results do not depend on it. */
     int32_t stack_entries;
 } ac_trace_params;
@@ -225,7 +228,8 @@ typedef struct ac_batch_config {
     int32_t chunk_rays;          /* rays per work item a warp takes from the queue; 0: default */
     int32_t grid_blocks;         /* persistent blocks; 0: SM count * occupancy */
     int32_t stack_entries;       /* traversal stack entries per lane (0: 32); at least every BVH scene's
-                                    bvh_stack_need, else AC_ERR_INVALID */
+                                    bvh_stack_need, else AC_ERR_INVALID (small AUTO rooms excepted,
+                                    see ac_trace_params::stack_entries) */
 } ac_batch_config;
 
 /* Band synthesis of J echograms (steam_rt.py:2205-2232, 3070-3083): per
@@ -369,7 +373,7 @@ typedef struct {
     int32_t block_size;          /* 0: 256 */
     int32_t chunk_rays;          /* rays a warp takes at a time (0: 64) */
     int32_t stack_entries;       /* traversal stack entries per lane (0: 32); a job whose scene needs more
-                                    (bvh_stack_need) is refused at submit */
+                                    (bvh_stack_need) is refused at submit, a small AUTO room scanned */
     int64_t idle_timeout_ns;     /* 0: 20 ms */
     int32_t reserve_blocks;      /* grid = blocks_per_sm * SMs - reserve_blocks: the SMs left one block short
                                     keep room for other kernels (band synthesis) beside the persistent launch */
