@@ -135,10 +135,10 @@ std::vector<Partition> partition_jobs(const ac_job *jobs, int32_t count) {
     return parts;
 }
 
-size_t partition_bytes(const ac_job *jobs, const Partition &part, const ac_batch_config *cfg) {
+size_t partition_bytes(const ac_job *jobs, const Partition &part, const ac_batch_config *cfg, bool copies) {
     const int32_t n = static_cast<int32_t>(part.indices.size());
     const size_t b = part.fp64 ? batch_workspace_bytes_f64(jobs, part.indices.data(), n, cfg)
-                               : batch_workspace_bytes_f32(jobs, part.indices.data(), n, cfg);
+                               : batch_workspace_bytes_f32(jobs, part.indices.data(), n, cfg, copies);
     return (b + 255) & ~static_cast<size_t>(255);
 }
 
@@ -227,7 +227,7 @@ int ac_batch_workspace_size(const ac_job *jobs, int32_t num_jobs, const ac_batch
     for (int32_t j = 0; j < num_jobs; ++j)
         if (!jobs[j].scene) return ac::fail(AC_ERR_INVALID, "job %d has no scene", j);
     size_t total = 0;
-    for (const ac::Partition &part : ac::partition_jobs(jobs, num_jobs)) total += ac::partition_bytes(jobs, part, config);
+    for (const ac::Partition &part : ac::partition_jobs(jobs, num_jobs)) total += ac::partition_bytes(jobs, part, config, true);
     *bytes = total;
     return AC_OK;
 }
@@ -244,9 +244,18 @@ int ac_trace_batch(const ac_job *jobs, int32_t num_jobs, const ac_batch_config *
         const int rc = ac::validate_trace(jobs[j].scene, &jobs[j].params, &jobs[j].outputs);
         if (rc != AC_OK) return ac::fail(rc, "job %d: %s", j, ac_last_error());
     }
-    size_t offset = 0;
-    for (const ac::Partition &part : ac::partition_jobs(jobs, num_jobs)) {
-        const size_t bytes = ac::partition_bytes(jobs, part, config);
+    const std::vector<ac::Partition> parts = ac::partition_jobs(jobs, num_jobs);
+    // copies of the accumulators only where the workspace holds those of every partition: one that was sized for a longer
+    // list, which has none or smaller ones, serves its parts too
+    std::vector<size_t> sizes;
+    size_t offset = 0, total = 0;
+    for (const ac::Partition &part : parts) {
+        sizes.push_back(ac::partition_bytes(jobs, part, config, true));
+        total += sizes.back();
+    }
+    for (size_t k = 0; k < parts.size(); ++k) {
+        const ac::Partition &part = parts[k];
+        const size_t bytes = total <= workspace_bytes ? sizes[k] : ac::partition_bytes(jobs, part, config, false);
         if (offset + bytes > workspace_bytes)
             return ac::fail(AC_ERR_CAPACITY, "batch workspace too small: %zu < %zu", workspace_bytes, offset + bytes);
         unsigned char *ws = static_cast<unsigned char *>(workspace) + offset;

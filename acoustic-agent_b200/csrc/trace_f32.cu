@@ -286,10 +286,11 @@ int launch_trace_f32(const ac_scene_s *scene, const ac_trace_params *p, const ac
     return AC_OK;
 }
 
-size_t batch_workspace_bytes_f32(const ac_job *jobs, const int32_t *indices, int32_t count, const ac_batch_config *) {
+size_t batch_workspace_bytes_f32(const ac_job *jobs, const int32_t *indices, int32_t count, const ac_batch_config *,
+                                 bool copies) {
     const std::vector<int32_t> order = scene_order(jobs, indices, count);
     const int64_t groups = count_groups(jobs, order);
-    return f32_layout(count, groups, shard_plan(jobs, order, groups, nullptr)).total;
+    return f32_layout(count, groups, copies ? shard_plan(jobs, order, groups, nullptr) : 0).total;
 }
 
 int launch_batch_f32(const ac_job *jobs_in, const int32_t *indices, int32_t count, const ac_batch_config *cfg,
@@ -299,7 +300,11 @@ int launch_batch_f32(const ac_job *jobs_in, const int32_t *indices, int32_t coun
     const std::vector<int32_t> order = scene_order(jobs_in, indices, count);
     const int64_t num_groups = count_groups(jobs_in, order);
     std::vector<int32_t> copies;
-    const size_t shard_words = shard_plan(jobs_in, order, num_groups, &copies);
+    size_t shard_words = shard_plan(jobs_in, order, num_groups, &copies);
+    if (f32_layout(count, num_groups, shard_words).total > workspace_bytes) {
+        shard_words = 0;
+        copies.assign(order.size(), 1);
+    }
     const F32Layout l = f32_layout(count, num_groups, shard_words);
     if (workspace_bytes < l.total)
         return fail(AC_ERR_CAPACITY, "batch workspace too small: %zu < %zu", workspace_bytes, l.total);
