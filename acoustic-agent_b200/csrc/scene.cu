@@ -42,8 +42,9 @@ struct Offsets {
 // 8-room apartment (52 walls, 374 boxes) BVH 5.1 ms < hybrid 6.3 < scan 9.6 (the last two by earlier kernels).
 constexpr int64_t kAutoBvhSurfaces = 16;
 constexpr int64_t kAutoHybridWalls = 16;
-// Float32 BVH node boxes are padded by this much (metres) beyond the surface bounds, or by 4e-7 of the largest
-// coordinate where that is more (beyond 250 m): a slab plane's t carries three float32 roundings of that size.
+// Float32 BVH node boxes are padded by this much (metres) beyond the surface bounds, or by 4e-7 of the scene's largest
+// coordinate where that is more (beyond 250 m): a slab plane's t carries three float32 roundings of the size of the box's
+// coordinates and the ray's.
 constexpr double kBvhPad = 1e-4, kBvhPadPerMetre = 4e-7;
 // Surfaces per BVH leaf unless the caller chooses: one surface per leaf measured
 // fastest on B200 for rooms of 30 to 430 surfaces (deeper tree, fewer tests).
@@ -472,8 +473,8 @@ extern "C" int ac_scene_create(const ac_scene_desc *d, ac_scene_t *out) {
                             (d->traversal == AC_TRAVERSAL_BVH || lists.hybrid ||
                              (d->traversal == AC_TRAVERSAL_AUTO && static_cast<int64_t>(members.size()) > kAutoBvhSurfaces));
             if (!lists.use_bvh) lists.hybrid = false;   // no boxes: plain scan
-            double reach = 0.0;
-            for (const int64_t i : members)
+            double reach = 0.0;   // of the whole scene: a hybrid tree's rays start on walls that it does not hold
+            for (int64_t i = 0; i < S; ++i)
                 for (int a = 0; a < 3; ++a)
                     reach = std::max({reach, std::fabs(blo[3 * i + a]), std::fabs(bhi[3 * i + a])});
             if (lists.use_bvh)
