@@ -308,17 +308,11 @@ __device__ __forceinline__ void service_finish(const FastTable &t, int slot, int
 // each (t = v * inv - o * inv); measured 2-4 % faster than (v - o) * inv on the
 // U room and the 8-room apartment, with identical results (node boxes are
 // padded, so the culling stays conservative under either rounding).
-#ifndef AC_FMA_SLAB
-#define AC_FMA_SLAB 1
-#endif
-
 struct FRay {
     float o[3];
     float d[3];
     float inv[3];
-#if AC_FMA_SLAB
     float oi[3];   // o * inv: a slab plane's t is then one fused multiply-add
-#endif
 };
 
 // Approximate reciprocal (MUFU, ~1 ulp): the float32 path needs no correctly rounded division.
@@ -339,19 +333,13 @@ __device__ __forceinline__ void make_ray(FRay &r, const float *o, const float *d
         r.o[a] = o[a];
         r.d[a] = d[a];
         r.inv[a] = safe_inv(d[a]);
-#if AC_FMA_SLAB
         r.oi[a] = o[a] * r.inv[a];
-#endif
     }
 }
 
 // t of the plane x_a = v along the ray (conservative box culling only: node boxes are padded)
 __device__ __forceinline__ float slab_t(const FRay &r, int a, float v) {
-#if AC_FMA_SLAB
     return fmaf(v, r.inv[a], -r.oi[a]);
-#else
-    return (v - r.o[a]) * r.inv[a];
-#endif
 }
 
 // Conservative slab test: could any point of the box be hit before max_t?
