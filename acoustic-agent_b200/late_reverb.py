@@ -359,12 +359,16 @@ class LateReverbRenderer:
         # (7.1 -> 3.2 ms with the kernels, 16 kHz).
         raw_at = raw.data_ptr() + 8 * (np.cumsum(lengths, dtype=np.uint64) - np.asarray(lengths, dtype=np.uint64))
         f = np.frombuffer(fdn_jobs, dtype=np.dtype(_lib.ACFdnJob))
-        f["absorptive"] = np.stack([d.absorptive for d in designs]).reshape(J, -1)
-        f["tone"] = np.stack([d.tone for d in designs]).reshape(J, -1)
-        f["delays"] = np.stack([d.delays for d in designs])
+        # whole rows of each field: a column of one value per job would be spread over the row
+        f["absorptive"] = np.stack([d.absorptive for d in designs]).reshape(J, NUM_LINES * 6 * 5)
+        f["tone"] = np.stack([d.tone for d in designs]).reshape(J, 6 * 5)
+        f["delays"] = np.stack([d.delays for d in designs]).reshape(J, NUM_LINES)
         f["allpass_delays"] = np.asarray([d.allpass for d in designs]).reshape(J, _lib.AC_FDN_ALLPASS)
         f["num_samples"] = lengths
-        f["preroll"] = f["delays"].max(axis=1) + f["allpass_delays"].sum(axis=1)
+        if all(type(d) is FdnDesign for d in designs):
+            f["preroll"] = f["delays"].max(axis=1) + f["allpass_delays"].sum(axis=1)
+        else:   # a caller's own design may start elsewhere
+            f["preroll"] = [d.preroll for d in designs]
         f["out"] = raw_at
         t = np.frombuffer(tail_jobs, dtype=np.dtype(_lib.ACLateTailJob))
         t["traced"], t["out"], t["fdn_component"] = np.asarray(addresses, dtype=np.uint64).T
@@ -374,7 +378,7 @@ class LateReverbRenderer:
         t["start"] = [w.start for w in wins]
         t["end"] = [w.end for w in wins]
         t["anchor"] = [[w.anchor(b) for b in range(6)] for w in wins]
-        t["changed_from"], t["num_samples"], t["bin_samples"], t["rate_index"] = np.asarray(scalars, dtype=np.int32).T
+        t["changed_from"], t["num_samples"], t["bin_samples"], t["rate_index"] = np.asarray(scalars, dtype=np.int64).astype(np.int32).T
         launch_stream = stream if stream is not None else torch.cuda.current_stream(self.device)
         if fdn_events is not None:
             fdn_events[0].record(launch_stream)
