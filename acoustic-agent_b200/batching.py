@@ -243,8 +243,9 @@ class RIRRenderer:
             plan.echo_prev.copy_(plan.echo_store)
             runtime.synthesize_batch(synth, plan.synth_workspace, stream=side, phase="raw")
             raw_done.record(side)
-            # the recursion's few blocks start before the trace takes every SM; the trace's persistent blocks
-            # that find no room beside them start when they end and take the chunks that are left then
+            # the recursion's blocks start before the trace takes every SM, a few in a small plan, more than the
+            # SMs hold in a large one; the trace's persistent blocks that find no room beside them start as they
+            # end and take the chunks that are left then
             runtime.synthesize_batch(synth, plan.synth_workspace, stream=side, phase="filter")
         main.wait_event(raw_done)
         with torch.cuda.stream(main):

@@ -37,9 +37,10 @@ struct Offsets {
 // Unless the caller chooses, a single room (at most kAutoHybridWalls walls) with any box traces in hybrid mode, its walls
 // in lockstep and its boxes in a BVH; other scenes of more than kAutoBvhSurfaces walls and boxes in BVH mode.  A room of no
 // more than kAutoBvhSurfaces never needs a stack: a launch with a shallower one than its tree needs scans it.  Measured on
-// B200: a 4-wall room, 10,000 / 400,000 rays: with 1 box scan 0.466 / 2.24 ms, hybrid 0.456 / 2.19, with 12 boxes scan
-// 0.668 / 2.60, hybrid 0.554 / 2.27, BVH 0.548 / 2.46; U room (8 walls, 20 boxes) hybrid 11.4 ms < BVH 11.8 < scan 12.3;
-// 8-room apartment (52 walls, 374 boxes) BVH 5.1 ms < hybrid 6.3 < scan 9.6 (the last two by earlier kernels).
+// B200, in batches: a 4-wall room, 10,000 / 400,000 rays x 60 bounces: with 1 box scan 0.465 / 2.12 ms, hybrid 0.445 /
+// 2.12, BVH 0.419 / 2.08, with 12 boxes scan 0.662 / 2.57, hybrid 0.546 / 2.28, BVH 0.545 / 2.47; U room (8 walls, 20
+// boxes), eight jobs of 200,000 rays, hybrid 8.24 ms, BVH 8.92, scan 10.4; 8-room apartment (52 walls, 303 boxes),
+// 1,000,000 rays, BVH 8.78 ms, hybrid 9.84, scan 17.4.
 constexpr int64_t kAutoBvhSurfaces = 16;
 constexpr int64_t kAutoHybridWalls = 16;
 // Float32 BVH node boxes are padded by this much (metres) beyond the surface bounds, or by 4e-7 of the scene's largest

@@ -356,7 +356,8 @@ class LateReverbRenderer:
             addresses.append((job.traced.data_ptr(), job.out.data_ptr(), job.component.data_ptr()))
             scalars.append((changed_from, N, max(1, int(round(float(job.bin_duration_s) * fs))), rate_index[fs]))
         # The tables are filled column by column: field by field through ctypes 256 jobs took 3 ms longer
-        # (7.1 -> 3.2 ms with the kernels, 16 kHz).
+        # (7.1 -> 3.2 ms with the kernels, 16 kHz, designs at hand; RT60s not seen before cost 0.9 ms per tail to
+        # design, see design_many).
         raw_at = raw.data_ptr() + 8 * (np.cumsum(lengths, dtype=np.uint64) - np.asarray(lengths, dtype=np.uint64))
         f = np.frombuffer(fdn_jobs, dtype=np.dtype(_lib.ACFdnJob))
         # whole rows of each field: a column of one value per job would be spread over the row

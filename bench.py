@@ -1719,12 +1719,12 @@ def l2_read_gbs(device) -> float:
 # SIMT efficiency (thread instructions per warp instruction / 32) and DRAM bytes per ray-bounce
 # (dram__bytes_read.sum + dram__bytes_write.sum of the captured launch over its ray-bounces).
 PROFILED = {
-    "u_room_20_boxes": {"issue_active": 0.6706, "simt_efficiency": 14.41 / 32.0,
-                        "dram_bytes_per_ray_bounce": (3123456 + 734208) / 52028160,
-                        "profile": "profiles/trace_kernel_u_room_20_boxes.md", "kernel_commit": "2860a90"},
-    "mixed_batch": {"issue_active": 0.6255, "simt_efficiency": 13.11 / 32.0,
-                    "dram_bytes_per_ray_bounce": (32922624 + 1248512) / 2209616616,
-                    "profile": "profiles/trace_kernel_mixed_batch_24_scenes.md", "kernel_commit": "2860a90"},
+    "u_room_20_boxes": {"issue_active": 0.6896, "simt_efficiency": 15.83 / 32.0,
+                        "dram_bytes_per_ray_bounce": (1478912 + 323584) / 52028160,
+                        "profile": "profiles/trace_kernel_u_room_20_boxes.md", "kernel_commit": "3609404"},
+    "mixed_batch": {"issue_active": 0.6942, "simt_efficiency": 13.63 / 32.0,
+                    "dram_bytes_per_ray_bounce": (4061440 + 1488640) / 2209616616,
+                    "profile": "profiles/trace_kernel_mixed_batch_24_scenes.md", "kernel_commit": "3609404"},
 }
 
 
