@@ -236,6 +236,15 @@ int64_t count_groups(const ac_job *jobs, const std::vector<int32_t> &order) {
     return groups;
 }
 
+// Warps per SM that a single job's rays are spread over.  In a small room whose sums lie in global memory the deposits of
+// more warps meet at the same addresses: a shoebox (scan) of 10,000 / 20,000 rays, 500 bins, takes 0.406 / 0.678 ms over
+// eight, 0.362 / 0.641 over two, a room of 6 boxes with 20,000 / 25,000 rays 0.638 / 0.827 over eight, 0.615 / 0.766 over
+// six; larger rooms' deposits are spread out (U room, 20,000 rays 0.498 over eight, 0.515 over six).
+int single_warps_per_sm(const ac_scene_s *scene, const FastScene &form, bool own_sums) {
+    if (own_sums || scene->num_surfaces > 24) return 8;
+    return form.num_bvh_nodes > 0 ? 6 : 2;
+}
+
 }  // namespace
 
 int launch_trace_f32(const ac_scene_s *scene, const ac_trace_params *p, const ac_trace_outputs *o, double scale,
@@ -255,16 +264,18 @@ int launch_trace_f32(const ac_scene_s *scene, const ac_trace_params *p, const ac
     }
     const int block = p->block_size > 0 ? p->block_size : kDefaultBlock;
     if (block % 32 != 0 || block > 256) return fail(AC_ERR_INVALID, "block_size must be a multiple of 32 up to 256");
-    FastTable table{};
-    table.lanes = p->grid_blocks > 0 ? 32 : warp_lanes(scene->device, p->num_rays, form.num_bvh_nodes > 0 ? 4 : 16);
-    table.chunk_rays = std::min(kDefaultChunkRays, table.lanes);
-    table.chunk_counter = reinterpret_cast<unsigned long long *>(o->counters) + 4;
     const int64_t cells = static_cast<int64_t>(kBands) * p->num_bins * (job.ambisonic_fx ? 4 : 1) + scene->num_surfaces;
     const int64_t sum_bytes = 4 * (4 * cells + 2 * scene->num_surfaces);
     const bool own_sums = sum_bytes <= kSharedSumBytes;
     // beside the sums no deeper stack than the tree uses, so that three blocks still fit an SM (U room, 400 bins, 100,000
     // rays: 0.98 ms with two, 0.72 with three; what lies above the need is never read)
     if (own_sums) entries = std::min(entries, stack_need(scene, form));
+    FastTable table{};
+    table.lanes = p->grid_blocks > 0 ? 32
+                                     : warp_lanes(scene->device, p->num_rays, form.num_bvh_nodes > 0 ? 4 : 16,
+                                                  single_warps_per_sm(scene, form, own_sums));
+    table.chunk_rays = std::min(kDefaultChunkRays, table.lanes);
+    table.chunk_counter = reinterpret_cast<unsigned long long *>(o->counters) + 4;
     const FastKernel kernel = pick_kernel<true>(p->rng_mode == AC_RNG_PHILOX, p->render_ambisonics != 0,
                                                 p->visual_limit > 0, own_sums, scene_is_lean(form));
     size_t smem = stack_smem_bytes(entries);
